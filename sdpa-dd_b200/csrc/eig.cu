@@ -1,404 +1,388 @@
 // Step-length eigenvalue lambda_min(L D L^T) per SDP block
 // (Jal::getMinEigen, sdpa_jordan.cpp:55-88):
-//   n > 20   Lanczos of Lal::getMinEigen (sdpa_linear.cpp:27-122) - same
-//            start vector, recurrences (Rtrmv/Rgemv/Rdot orders), checkpoint
-//            and stopping rules; the k x k tridiagonal eigenproblem at a
-//            checkpoint is solved for its smallest eigenpair by Sturm
-//            multisection over 15 warps plus inverse iteration (the reference uses
-//            implicit QR, Rsteqr; both give the eigenvalue and the last
-//            eigenvector component to dd rounding).
+//   n > 20   Lanczos of Lal::getMinEigen (sdpa_linear.cpp:27-122): same start
+//            vector, recurrences, checkpoint and stopping rules.  The sums of
+//            the three matrix-vector products and the two dot products run
+//            split over lanes, warps and the CTAs of a cluster (the
+//            reference's own sums follow its OpenMP threads); the k x k
+//            tridiagonal eigenproblem of a checkpoint is tri_eig.cuh's (the
+//            reference uses implicit QR, Rsteqr; both give the eigenvalue
+//            and the last eigenvector component to dd rounding).
 //   n <= 20  M = L (D L^T) by two Rgemm, then the smallest eigenvalue of the
 //            lower triangle of M (the reference's Rsyev "N","L") by
-//            Householder tridiagonalisation (one warp) and Sturm multisection.
-// The whole Lanczos loop runs in one CTA per block: no host round trip per
-// step.
+//            Householder tridiagonalisation (one warp) and tri_eig.cuh.
+// The whole Lanczos loop runs in one cluster per block: no host round trip
+// per step.
 #include "newton.h"
+
+#include <algorithm>
+
+#include <cooperative_groups.h>
 
 #include "blas.h"
 #include "devops.cuh"
 #include "eig_kernels.cuh"
 #include "prof.h"
+#include "tri_eig.cuh"
 
 namespace sddd {
+
+namespace cg = cooperative_groups;
 
 // QD double-vs-dd comparisons (dd_inline.h operator< / operator>)
 __device__ __forceinline__ bool d_lt_dd(double a, dd_t b) { return a < b.hi || (a == b.hi && b.lo > 0.0); }
 __device__ __forceinline__ bool d_gt_dd(double a, dd_t b) { return a > b.hi || (a == b.hi && b.lo < 0.0); }
 
-// Number of eigenvalues of tridiagonal (d, e2 = e^2) below x.
-__device__ int sturm_count(int k, const dd_t *d, const dd_t *e2, dd_t x) {
-    int c = 0;
-    dd_t q = dd_sub(d[0], x);
-    if (q.hi < 0.0) c++;
-    for (int i = 1; i < k; ++i) {
-        if (dd_is_zero(q)) q = dd_make(1e-300, 0.0);
-        q = dd_sub(dd_sub(d[i], x), dd_div(e2[i - 1], q));
-        if (q.hi < 0.0) c++;
-    }
-    return c;
-}
+namespace {
 
-// The same count on the high parts in double: a quick estimate only.
-__device__ int sturm_count_d(int k, const dd_t *d, const dd_t *e2, double x) {
-    int c = 0;
-    double q = d[0].hi - x;
-    if (q < 0.0) c++;
-    for (int i = 1; i < k; ++i) {
-        if (q == 0.0) q = 1e-300;
-        q = (d[i].hi - x) - e2[i - 1].hi / q;
-        if (q < 0.0) c++;
-    }
-    return c;
-}
+constexpr int LZ_WARPS = LZ_THREADS / 32;
+constexpr int LZ_CHUNK = 8;     // rows a warp takes together
+constexpr int LZ_CLUSTER = 16;  // most CTAs of a cluster
 
-// Smallest eigenvalue of the k x k tridiagonal (d, e) by multisection over
-// the lanes of nw warps (warps 0 .. nw-1 of the CTA, all of their threads
-// calling; nw = 1 runs on one warp alone); every thread returns the same
-// value.  A first multisection in double on the high parts narrows the
-// Gershgorin bracket to ~2^-40 of the spectrum's scale; that bracket is
-// kept only when dd Sturm counts confirm it (no eigenvalue below its lower
-// end, one below its upper end), and the dd multisection then runs from it.
-// P = 32 nw points a round; each warp's ballot goes to shared memory (ball:
-// 2 nw + 2 words, two alternating halves), so that every thread finds the
-// first point with a non-zero count.
-__device__ dd_t tri_min_eigenvalue(int k, const dd_t *d, const dd_t *e, dd_t *e2, int nw, unsigned *ball) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = threadIdx.x, P = 32 * nw;
-    auto sync = [&]() {
-        if (nw == 1)
-            __syncwarp();
-        else
-            asm volatile("bar.sync 1, %0;" ::"r"(P) : "memory");
-    };
-    // index of the first point (over all warps) whose flag is set, or -1
-    int half = 0;
-    auto first_set = [&](bool flag) {
-        const unsigned b = __ballot_sync(0xffffffffu, flag);
-        unsigned *hb = ball + half * nw;
-        if (lane == 0) hb[warp] = b;
-        sync();
-        int first = -1;
-        for (int w = 0; w < nw; ++w)
-            if (hb[w] != 0u) {
-                first = 32 * w + __ffs(hb[w]) - 1;
-                break;
-            }
-        half ^= 1; // the next round writes the other half: no second barrier
-        return first;
-    };
-    dd_t lo = d[0], hi = d[0];
-    for (int i = 0; i < k; ++i) {
-        dd_t r = dd_zero();
-        if (i > 0) r = dd_add(r, dd_abs(e[i - 1]));
-        if (i + 1 < k) r = dd_add(r, dd_abs(e[i]));
-        dd_t a = dd_sub(d[i], r), b = dd_add(d[i], r);
-        if (dd_lt(a, lo)) lo = a;
-        if (dd_gt(b, hi)) hi = b;
+// Compensated dot product of dd operands (Ogita, Rump and Oishi's Dot2 with
+// the operands' low parts in the error term): the running sum's chain is one
+// addition a term, twelve FP64 operations against dd_acc(dd_mul)'s twenty,
+// and the sum is as if rounded once from twice the working precision.
+struct DotAcc {
+    double s = 0.0, e = 0.0;
+    __device__ __forceinline__ void term(double2 a, double2 b) {
+        const double p = __dmul_rn(a.x, b.x);
+        double pe = __fma_rn(a.x, b.x, -p);
+        pe = __fma_rn(a.x, b.y, pe);
+        pe = __fma_rn(a.y, b.x, pe);
+        double se;
+        s = ddm::two_sum(s, p, se);
+        e = __dadd_rn(e, __dadd_rn(pe, se));
     }
-    if (g == 0)
-        for (int i = 0; i + 1 < k; ++i) e2[i] = dd_mul(e[i], e[i]);
-    sync();
-    dd_t w = dd_sub(hi, lo);
-    lo = dd_sub(lo, dd_mul_d(w, 1e-10));
-    hi = dd_add(hi, dd_mul_d(w, 1e-10));
-    const double PP = (double)(P + 1);
-    {
-        double dlo = lo.hi, dhi = hi.hi;
-        for (int round = 0; round < 12; ++round) {
-            const double width = dhi - dlo;
-            const double x = dlo + width * (double)(g + 1) / PP;
-            const bool below = !(x > dlo) ? false : !(x < dhi) ? true : sturm_count_d(k, d, e2, x) >= 1;
-            const int first = first_set(below);
-            double nlo, nhi;
-            if (first < 0) {
-                nlo = dlo + width * (double)P / PP;
-                nhi = dhi;
-            } else {
-                nhi = dlo + width * (double)(first + 1) / PP;
-                nlo = first == 0 ? dlo : dlo + width * (double)first / PP;
-            }
-            if (!(nlo < nhi) || (nlo == dlo && nhi == dhi)) break;
-            dlo = nlo;
-            dhi = nhi;
-        }
-        const double rad = (fabs(lo.hi) + fabs(hi.hi) + (hi.hi - lo.hi)) * 0x1p-40;
-        const dd_t blo = dd_max(lo, dd_from(dlo - rad)), bhi = dd_min(hi, dd_from(dhi + rad));
-        bool bad = false;
-        if (g == 0) bad = sturm_count(k, d, e2, blo) != 0;
-        if (g == 1) bad = !(dd_lt(blo, bhi) && sturm_count(k, d, e2, bhi) >= 1);
-        if (first_set(bad) < 0) {
-            lo = blo;
-            hi = bhi;
-        }
+    __device__ __forceinline__ dd_t value() const {
+        double lo, hi = ddm::fast_two_sum(s, e, lo);
+        return dd_make(hi, lo);
     }
-    for (int round = 0; round < 40; ++round) {
-        const dd_t width = dd_sub(hi, lo);
-        // P interior points x_g = lo + width (g+1)/(P+1); the smallest
-        // eigenvalue lies below the first x with a non-zero Sturm count,
-        // or above x_(P-1) when there is none.
-        const dd_t x = dd_add(lo, dd_div_d(dd_mul_d(width, (double)(g + 1)), PP));
-        bool below;
-        if (!dd_gt(x, lo))
-            below = false;
-        else if (!dd_lt(x, hi))
-            below = true;
-        else
-            below = sturm_count(k, d, e2, x) >= 1;
-        const int first = first_set(below);
-        dd_t nlo, nhi;
-        if (first < 0) {
-            nlo = dd_add(lo, dd_div_d(dd_mul_d(width, (double)P), PP));
-            nhi = hi;
-        } else {
-            nhi = dd_add(lo, dd_div_d(dd_mul_d(width, (double)(first + 1)), PP));
-            nlo = first == 0 ? lo : dd_add(lo, dd_div_d(dd_mul_d(width, (double)first), PP));
-        }
-        if (!dd_lt(nlo, nhi) || (dd_eq(nlo, lo) && dd_eq(nhi, hi))) break;
-        lo = nlo;
-        hi = nhi;
-    }
-    return dd_mul_d(dd_add(lo, hi), 0.5);
-}
-
-// Last component of the unit eigenvector of (d, e) for eigenvalue l:
-// three steps of inverse iteration with a partially pivoted tridiagonal
-// solve (single thread; k <= LZ_KMAX).  T - l I is factored once; each
-// step solves with the factors.
-__device__ dd_t tri_last_component(int k, const dd_t *d, const dd_t *e, dd_t l, dd_t tnorm, dd_t *v, dd_t *dd_, dd_t *du, dd_t *du2, dd_t *dl, int *piv) {
-    for (int i = 0; i < k; ++i) v[i] = dd_from(1.0);
-    {
-        for (int i = 0; i < k; ++i) {
-            dd_[i] = dd_sub(d[i], l);
-            du[i] = (i + 1 < k) ? e[i] : dd_zero();
-            dl[i] = (i + 1 < k) ? e[i] : dd_zero();
-            du2[i] = dd_zero();
-        }
-        for (int i = 0; i + 1 < k; ++i) {
-            if (!dd_lt(dd_abs(dd_[i]), dd_abs(dl[i]))) {
-                piv[i] = 0;
-                if (dd_is_zero(dd_[i])) dd_[i] = dd_mul_d(tnorm, 1e-32);
-                dd_t f = dd_div(dl[i], dd_[i]);
-                dl[i] = f;
-                dd_[i + 1] = dd_sub(dd_[i + 1], dd_mul(f, du[i]));
-            } else {
-                piv[i] = 1;
-                dd_t f = dd_div(dd_[i], dl[i]);
-                dd_[i] = dl[i];
-                dl[i] = f;
-                dd_t t = du[i];
-                du[i] = dd_[i + 1];
-                dd_[i + 1] = dd_sub(t, dd_mul(f, dd_[i + 1]));
-                if (i + 2 < k) {
-                    du2[i] = du[i + 1];
-                    du[i + 1] = dd_neg(dd_mul(f, du[i + 1]));
-                }
-            }
-        }
-        if (dd_is_zero(dd_[k - 1])) dd_[k - 1] = dd_mul_d(tnorm, 1e-32);
-    }
-    for (int it = 0; it < 3; ++it) {
-        for (int i = 0; i + 1 < k; ++i) {
-            if (piv[i]) {
-                dd_t t = v[i];
-                v[i] = v[i + 1];
-                v[i + 1] = dd_sub(t, dd_mul(dl[i], v[i + 1]));
-            } else {
-                v[i + 1] = dd_sub(v[i + 1], dd_mul(dl[i], v[i]));
-            }
-        }
-        for (int i = k - 1; i >= 0; --i) {
-            dd_t t = v[i];
-            if (i + 1 < k) t = dd_sub(t, dd_mul(du[i], v[i + 1]));
-            if (i + 2 < k) t = dd_sub(t, dd_mul(du2[i], v[i + 2]));
-            v[i] = dd_div(t, dd_[i]);
-        }
-        dd_t nrm = dd_zero();
-        for (int i = 0; i < k; ++i) nrm = dd_acc(nrm, dd_mul(v[i], v[i]));
-        nrm = dd_sqrt(nrm);
-        for (int i = 0; i < k; ++i) v[i] = dd_div(v[i], nrm);
-    }
-    return v[k - 1];
-}
-
-// Warps of the Lanczos CTA that run the checkpoint's multisection; the last
-// warp's lane 0 computes r.r beside them.
-constexpr int LZ_EIG_WARPS = LZ_THREADS / 32 - 1;
-struct LanczosShared {
-    dd_t diag[LZ_KMAX], off[LZ_KMAX], e2[LZ_KMAX];
-    unsigned ball[2 * LZ_EIG_WARPS + 2];
-    dd_t v[LZ_KMAX], t0[LZ_KMAX], t1[LZ_KMAX], t2[LZ_KMAX], t3[LZ_KMAX];
-    int piv[LZ_KMAX];
-    dd_t alpha, beta, value, mn, mn_old, err, rr;
-    int go, check;
 };
 
-// One CTA per block: work holds 5 n-vectors (q, qold, r, w, tmp).  With a
-// second space (Lsp2, Dsp2), CTAs nb.. take the same blocks of that space,
-// so the two step-length eigenvalues run side by side.
+struct alignas(16) LanczosShared {
+    dd_t diag[LZ_KMAX], off[LZ_KMAX], ioff[LZ_KMAX];
+    TriWork<LZ_KMAX, LZ_WARPS> tri;
+    dd_t psum[LZ_WARPS * LZ_CHUNK];
+    dd_t pa[LZ_CLUSTER], pr[LZ_CLUSTER];
+};
+
+// A vector the products read: in shared memory (every CTA holds all of it),
+// or, for orders whose vectors do not fit there, in global memory (read past
+// L1, which is not coherent between the CTAs).
+template <bool SMEM> __device__ __forceinline__ double2 lz_ld(const dd_t *v, long i) {
+    const double2 *p = reinterpret_cast<const double2 *>(v) + i;
+    return SMEM ? *p : __ldcg(p);
+}
+__device__ __forceinline__ double2 mat_ld(const dd_t *p) { return __ldg(reinterpret_cast<const double2 *>(p)); }
+
+// Eight rows i0 .. i0+7 of a product with v, part `part` of 2^lp of the
+// terms: lane (row, phase) takes every (4 2^lp)-th term.  FULL: rows of M v;
+// LOWER: of M's lower triangle; LOWER_T: of its transpose (row i is column i
+// from the diagonal down).  A load instruction covers 128 contiguous bytes of
+// each of 4 columns (LOWER_T: 64 bytes of each of 8, the rest of the line at
+// the next step).  Every lane of a row returns the part's sum.
+enum { LZ_FULL, LZ_LOWER, LZ_LOWER_T };
+template <int FORM, bool SMEM> __device__ __forceinline__ dd_t lz_rows(const dd_t *M, int n, int i0, int part, int lp, const dd_t *v) {
+    const int lane = threadIdx.x & 31, i = i0 + (lane & 7), step = 4 << lp;
+    const int end = i >= n ? 0 : FORM == LZ_LOWER ? i + 1 : n;
+    const long sj = FORM == LZ_LOWER_T ? 1 : n; // from one term to the next
+    const dd_t *Mi = FORM == LZ_LOWER_T ? M + (long)n * i : M + i;
+    DotAcc acc;
+    int j = part * 4 + (lane >> 3);
+    if (FORM == LZ_LOWER_T) j += i0;
+    // the loads of eight terms in flight, then of two
+    for (; j + 7 * step < end; j += 8 * step) {
+        double2 a[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int ju = j + u * step;
+            a[u] = FORM == LZ_LOWER_T && ju < i ? make_double2(0.0, 0.0) : mat_ld(Mi + sj * ju);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc.term(a[u], lz_ld<SMEM>(v, j + u * step));
+    }
+    for (; j + step < end; j += 2 * step) {
+        const double2 a0 = FORM == LZ_LOWER_T && j < i ? make_double2(0.0, 0.0) : mat_ld(Mi + sj * j);
+        const double2 a1 = FORM == LZ_LOWER_T && j + step < i ? make_double2(0.0, 0.0) : mat_ld(Mi + sj * (j + step));
+        acc.term(a0, lz_ld<SMEM>(v, j));
+        acc.term(a1, lz_ld<SMEM>(v, j + step));
+    }
+    for (; j < end; j += step)
+        if (FORM != LZ_LOWER_T || j >= i) acc.term(mat_ld(Mi + sj * j), lz_ld<SMEM>(v, j));
+    dd_t t = acc.value();
+    t = dd_add(t, shfl_xor_dd(t, 8));
+    return dd_add(t, shfl_xor_dd(t, 16));
+}
+
+// The Lanczos loop of one block by one cluster: CTA r of R owns the 8-row
+// chunks r, r + R, ... (the triangular products' work then spreads evenly),
+// forms those rows of each product and stores them into every CTA's copy of
+// the vector; four cluster barriers a step (after w = L^T q, tmp = X w,
+// w = L tmp with the parts of q.w, and r with the parts of r.r).  Every CTA
+// holds the same scalars, bit for bit (the same operations on the same
+// values), so the CTAs agree on every branch without a broadcast.
+// Bound by latency up to n of about 200 (barriers, the folds of partial sums
+// and the checkpoints' tridiagonal solves, 9 - 12 us each), by the L2 reads
+// of one GPC beyond.  One CTA whose threads each ran a row's whole chain of n
+// dependent dd sums took 1.20 / 1.98 / 3.73 / 10.6 / 24.1 ms at n = 30 / 100
+// / 200 / 500 / 777 (random L D L^T, 16 to 38 steps); this form 0.24 / 0.34 /
+// 0.45 / 0.88 / 1.74 ms.
+template <bool SMEM>
 __global__ void __launch_bounds__(LZ_THREADS) lanczos_kernel(const int *blk_ids, int nb, const int *sizes, const long *off, const dd_t *Lsp,
                                                              const dd_t *Dsp, const dd_t *Lsp2, const dd_t *Dsp2, dd_t *work, long work_stride, dd_t *out) {
-    __shared__ LanczosShared S;
-    const bool second = (int)blockIdx.x >= nb;
-    const int b = blk_ids[second ? blockIdx.x - nb : blockIdx.x];
-    if (second) {
-        Lsp = Lsp2;
-        Dsp = Dsp2;
-    }
+    extern __shared__ double2 lz_smem[];
+    LanczosShared &S = *reinterpret_cast<LanczosShared *>(lz_smem);
+    cg::cluster_group cl = cg::this_cluster();
+    const int R = (int)cl.num_blocks(), rank = (int)cl.block_rank(), cid = (int)blockIdx.x / R;
+    const bool second = cid >= nb;
+    const int b = blk_ids[second ? cid - nb : cid];
     const int n = sizes[b];
-    const dd_t *L = Lsp + off[b], *X = Dsp + off[b];
-    dd_t *q = work + blockIdx.x * work_stride, *qold = q + n, *r = qold + n, *w = r + n, *tmp = w + n;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    for (int i = tid; i < n; i += nt) {
-        st_dd(q + i, dd_zero());
-        st_dd(r + i, dd_from(1.0));
+    const dd_t *L = (second ? Lsp2 : Lsp) + off[b], *X = (second ? Dsp2 : Dsp) + off[b];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int chunks = (n + LZ_CHUNK - 1) / LZ_CHUNK;
+    const int nch = rank < chunks ? (chunks - rank - 1) / R + 1 : 0, nown = nch * LZ_CHUNK;
+    // q, w and tmp (tmp also carries r between the steps), then this CTA's
+    // rows of w and of the previous q
+    dd_t *local = reinterpret_cast<dd_t *>(&S + 1), *q, *w, *tmp, *wl, *ql;
+    if (SMEM) {
+        q = local, w = q + n, tmp = w + n, wl = tmp + n, ql = wl + (chunks + R - 1) / R * LZ_CHUNK;
+    } else {
+        q = work + (long)cid * work_stride, w = q + n, tmp = w + n;
+        wl = local, ql = wl + (chunks + R - 1) / R * LZ_CHUNK;
     }
-    if (tid == 0) {
-        S.mn = dd_from(1.0e+51);
-        S.mn_old = dd_from(1.0e+52);
-        S.err = dd_from(1.0e+10);
-        S.beta = dd_sqrt(dd_from((double)n));
+    // global row of own slot s (may be >= n in the last chunk)
+    auto row_of = [&](int s) { return (rank + R * (s >> 3)) * LZ_CHUNK + (s & 7); };
+    // value x of row i into every CTA's copy of v; lanes p of P share the copies
+    auto emit = [&](dd_t *v, int i, dd_t x, int p, int P) {
+        if (i >= n) return;
+        if (SMEM) {
+            for (int d = p; d < R; d += P) *cl.map_shared_rank(reinterpret_cast<double2 *>(v) + i, d) = make_double2(x.hi, x.lo);
+        } else if (p == 0) {
+            __stcg(reinterpret_cast<double2 *>(v) + i, make_double2(x.hi, x.lo));
+        }
+    };
+    // few own chunks: 2, 4, 8 or 16 warps share a chunk's terms
+    int lp = 0;
+    while (nch > 0 && (2 << lp) * nch <= LZ_WARPS) ++lp;
+    const int part = warp & ((1 << lp) - 1);
+    // one product: rows of this CTA's chunks, summed over the parts, to v
+    // (wl when v is null)
+    auto product = [&](auto &&chunk, dd_t *v) {
+        for (int s = warp >> lp; s < nch; s += LZ_WARPS >> lp) {
+            const dd_t t = chunk((rank + R * s) * LZ_CHUNK);
+            const int row = lane & 7, p = lane >> 3;
+            if (lp > 0) {
+                if (p == 0) S.psum[((s * LZ_CHUNK + row) << lp) + part] = t;
+            } else if (v) {
+                emit(v, (rank + R * s) * LZ_CHUNK + row, t, p, 4);
+            } else if (p == 0) {
+                wl[s * LZ_CHUNK + row] = t;
+            }
+        }
+        if (lp > 0) {
+            __syncthreads();
+            const int live = nown << lp; // at most 128, whole groups of 2^lp lanes
+            if (tid < live) {
+                const int left = live - warp * 32;
+                const unsigned mask = left >= 32 ? 0xffffffffu : (1u << left) - 1u;
+                dd_t t = S.psum[tid];
+                for (int m = 1; m < 1 << lp; m <<= 1)
+                    t = dd_add(t, dd_make(__shfl_xor_sync(mask, t.hi, m), __shfl_xor_sync(mask, t.lo, m)));
+                const int s = tid >> lp, p = tid & ((1 << lp) - 1);
+                if (v)
+                    emit(v, row_of(s), t, p, 1 << lp);
+                else if (p == 0)
+                    wl[s] = t;
+            }
+        }
+    };
+    // sum of the CTAs' parts, the same in every thread
+    auto gather = [&](const dd_t *p) {
+        dd_t t = lane < R ? p[lane] : dd_zero();
+        for (int m = 1; m < R; m <<= 1) t = dd_add(t, shfl_xor_dd(t, m));
+        return shfl_dd(t, 0);
+    };
+
+    for (int i = tid; i < n; i += LZ_THREADS) {
+        if (SMEM || rank == 0) {
+            st_dd(q + i, dd_zero());
+            st_dd(tmp + i, dd_from(1.0));
+        }
     }
-    __syncthreads();
-    const dd_t sqn10 = dd_add_d(dd_sqrt(dd_from((double)n)), 10.0);
+    for (int s = tid; s < nown; s += LZ_THREADS) ql[s] = dd_zero();
+    dd_t mn = dd_from(1.0e+51), mn_old = dd_from(1.0e+52), err = dd_from(1.0e+10), beta = dd_sqrt(dd_from((double)n));
+    dd_t value = dd_div(dd_from(1.0), beta); // 1 / beta
+    const dd_t sqn10 = dd_add_d(beta, 10.0);
     const dd_t sqn9 = dd_sqrt(dd_add_d(dd_from((double)n), 9.0));
+    cl.sync();
     int k = 0, kk = 0;
     while (true) {
-        if (tid == 0) {
-            const dd_t mn = S.mn, mo = S.mn_old;
-            bool c1 = dd_gt(dd_abs(dd_sub(mn, mo)), dd_add_d(dd_mul_d(dd_abs(mn), 1.0e-5), 1.0e-8));
-            bool c2 = dd_gt(dd_abs(dd_mul(S.err, S.beta)), dd_add_d(dd_mul_d(dd_abs(mn), 1.0e-2), 1.0e-4));
-            S.go = (k < n && k < LZ_KMAX && d_lt_dd((double)k, sqn10) && dd_gt_d(S.beta, 1.0e-16) && (c1 || c2)) ? 1 : 0;
-            S.value = dd_div(dd_from(1.0), S.beta);
-        }
-        __syncthreads();
-        if (!S.go) break;
-        const dd_t value = S.value;
+        const bool c1 = dd_gt(dd_abs(dd_sub(mn, mn_old)), dd_add_d(dd_mul_d(dd_abs(mn), 1.0e-5), 1.0e-8));
+        const bool c2 = dd_gt(dd_abs(dd_mul(err, beta)), dd_add_d(dd_mul_d(dd_abs(mn), 1.0e-2), 1.0e-4));
+        if (!(k < n && k < LZ_KMAX && d_lt_dd((double)k, sqn10) && dd_gt_d(beta, 1.0e-16) && (c1 || c2))) break;
+        if (tid == 0 && k > 0) S.ioff[k - 1] = value;
         // qold = q; q = r * value (Rcopy + Rscal)
-        for (int i = tid; i < n; i += nt) {
-            st_dd(qold + i, ld_dd(q + i));
-            dd_t qi = dd_mul(value, ld_dd(r + i));
-            st_dd(q + i, qi);
+        for (int s = tid; s < nown; s += LZ_THREADS) {
+            const int i = row_of(s);
+            if (i < n && k > 0) {
+                const double2 x = lz_ld<SMEM>(q, i);
+                ql[s] = dd_make(x.x, x.y);
+            }
         }
-        __syncthreads();
-        // Each product below is a sequential chain per entry; the loads of
-        // eight steps go out ahead of their terms (same order of the sums).
+        if (SMEM) {
+            __syncthreads();
+            for (int i = tid; i < n; i += LZ_THREADS) st_dd(q + i, dd_mul(value, ld_dd(tmp + i)));
+            __syncthreads();
+        } else {
+            for (int s = tid; s < nown; s += LZ_THREADS) {
+                const int i = row_of(s);
+                if (i < n) {
+                    const double2 x = __ldcg(reinterpret_cast<const double2 *>(tmp) + i);
+                    emit(q, i, dd_mul(value, dd_make(x.x, x.y)), 0, 1);
+                }
+            }
+            cl.sync();
+        }
         // w = L^T q (Rtrmv "Lower","Transpose")
-        for (int j = tid; j < n; j += nt) {
-            const dd_t *Lc = L + (long)n * j;
-            dd_t t = dd_mul(ld_dd(q + j), ld_dd(Lc + j));
-            int i = j + 1;
-            for (; i + 8 <= n; i += 8) {
-                dd_t a[8], b[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    a[u] = ld_dd(Lc + i + u);
-                    b[u] = ld_dd(q + i + u);
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) t = dd_acc(t, dd_mul(a[u], b[u]));
-            }
-            for (; i < n; ++i) t = dd_acc(t, dd_mul(ld_dd(Lc + i), ld_dd(q + i)));
-            st_dd(w + j, t);
-        }
-        __syncthreads();
+        product([&](int i0) { return lz_rows<LZ_LOWER_T, SMEM>(L, n, i0, part, lp, q); }, w);
+        cl.sync();
         // tmp = X w (Rgemv "N", alpha 1, beta 0)
-        for (int i = tid; i < n; i += nt) {
-            dd_t t = dd_zero();
-            int j = 0;
-            for (; j + 8 <= n; j += 8) {
-                dd_t a[8], b[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    a[u] = ld_dd(w + j + u);
-                    b[u] = ld_dd(X + i + (long)n * (j + u));
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) t = dd_acc(t, dd_mul(dd_mul(dd_from(1.0), a[u]), b[u]));
+        product([&](int i0) { return lz_rows<LZ_FULL, SMEM>(X, n, i0, part, lp, w); }, tmp);
+        cl.sync();
+        // w = L tmp (Rtrmv "Lower","NoTranspose"): own rows, and their part of
+        // alpha = q.w
+        product([&](int i0) { return lz_rows<LZ_LOWER, SMEM>(L, n, i0, part, lp, tmp); }, nullptr);
+        __syncthreads();
+        if (warp == 0) {
+            DotAcc acc;
+            for (int s = lane; s < nown; s += 32) {
+                const int i = row_of(s);
+                if (i < n) acc.term(lz_ld<SMEM>(q, i), make_double2(wl[s].hi, wl[s].lo));
             }
-            for (; j < n; ++j) t = dd_acc(t, dd_mul(dd_mul(dd_from(1.0), ld_dd(w + j)), ld_dd(X + i + (long)n * j)));
-            st_dd(tmp + i, t);
+            const dd_t t = warp_sum_dd(acc.value());
+            if (lane < R) *cl.map_shared_rank(&S.pa[rank], lane) = t;
         }
-        __syncthreads();
-        // w = L tmp (Rtrmv "Lower","NoTranspose": row i, j descending)
-        for (int i = tid; i < n; i += nt) {
-            dd_t t = dd_mul(ld_dd(tmp + i), ld_dd(L + i + (long)n * i));
-            int j = i - 1;
-            for (; j >= 7; j -= 8) {
-                dd_t a[8], b[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    a[u] = ld_dd(tmp + j - u);
-                    b[u] = ld_dd(L + i + (long)n * (j - u));
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (!dd_is_zero(a[u])) t = dd_acc(t, dd_mul(a[u], b[u]));
+        cl.sync();
+        const dd_t alpha = gather(S.pa);
+        if (tid == 0) S.diag[k] = alpha;
+        // r = w - alpha q - beta qold (Rcopy, Raxpy, Raxpy), own rows, and
+        // their part of r.r
+        if (warp == 0) {
+            const dd_t ma = dd_neg(alpha), mb = dd_neg(beta);
+            DotAcc acc;
+            for (int s = lane; s < nown; s += 32) {
+                const int i = row_of(s);
+                if (i >= n) continue;
+                const double2 qi = lz_ld<SMEM>(q, i);
+                dd_t ri = dd_acc(wl[s], dd_mul(ma, dd_make(qi.x, qi.y)));
+                ri = dd_acc(ri, dd_mul(mb, ql[s]));
+                acc.term(make_double2(ri.hi, ri.lo), make_double2(ri.hi, ri.lo));
+                emit(tmp, i, ri, 0, 1);
             }
-            for (; j >= 0; --j) {
-                dd_t xj = ld_dd(tmp + j);
-                if (!dd_is_zero(xj)) t = dd_acc(t, dd_mul(xj, ld_dd(L + i + (long)n * j)));
-            }
-            st_dd(w + i, t);
+            const dd_t t = warp_sum_dd(acc.value());
+            if (lane < R) *cl.map_shared_rank(&S.pr[rank], lane) = t;
         }
-        __syncthreads();
-        if (tid == 0) {
-            S.alpha = seq_dot(n, q, w);
-            S.diag[k] = S.alpha;
+        cl.sync();
+        {
+            // 1/beta and beta from one reciprocal square root and a Newton step
+            const dd_t rr = gather(S.pr);
+            const double x = rsqrt(rr.hi);
+            const dd_t t = dd_mul(rr, dd_sqr_d(x));
+            value = dd_add_dd_exact(x, 0.5 * x * ((1.0 - t.hi) - t.lo));
+            beta = dd_mul(rr, value);
+            if (!(rr.hi > 0.0)) beta = dd_sqrt(rr); // zero or not a number: the loop ends
         }
-        __syncthreads();
-        const dd_t ma = dd_neg(S.alpha), mb = dd_neg(S.beta);
-        // r = w - alpha q - beta qold (Rcopy, Raxpy, Raxpy)
-        for (int i = tid; i < n; i += nt) {
-            dd_t ri = ld_dd(w + i);
-            if (!dd_is_zero(ma)) ri = dd_acc(ri, dd_mul(ma, ld_dd(q + i)));
-            if (!dd_is_zero(mb)) ri = dd_acc(ri, dd_mul(mb, ld_dd(qold + i)));
-            st_dd(r + i, ri);
-        }
-        __syncthreads();
+        if (tid == 0) S.off[k] = beta;
         // checkpoint: kk >= sqrt(k) || k == n-1 || k > sqrt(n+9)
-        const dd_t sk = dd_sqrt(dd_from((double)k));
-        const bool check = dd_le_d(sk, (double)kk) || k == n - 1 || d_gt_dd((double)k, sqn9);
-        if (check) {
+        if (dd_le_d(dd_sqrt(dd_from((double)k)), (double)kk) || k == n - 1 || d_gt_dd((double)k, sqn9)) {
             kk = 0;
-            if (tid < 32 * LZ_EIG_WARPS) {
-                dd_t lam = tri_min_eigenvalue(k + 1, S.diag, S.off, S.e2, LZ_EIG_WARPS, S.ball);
-                if (tid == 0) {
-                    dd_t lo = S.diag[0], hi = S.diag[0];
-                    for (int i = 0; i <= k; ++i) {
-                        lo = dd_min(lo, S.diag[i]);
-                        hi = dd_max(hi, S.diag[i]);
-                    }
-                    dd_t tnorm = dd_add(dd_add(dd_abs(lo), dd_abs(hi)), dd_from(1e-300));
-                    dd_t last = tri_last_component(k + 1, S.diag, S.off, lam, tnorm, S.v, S.t0, S.t1, S.t2, S.t3, S.piv);
-                    S.mn_old = S.mn;
-                    S.mn = lam;
-                    S.err = last;
-                }
-            }
+            mn_old = mn;
+            tri_min_eigenpair<LZ_KMAX, LZ_WARPS>(k + 1, S.diag, S.off, S.ioff, S.tri, mn, err);
         }
-        // r.r on the last warp, beside the checkpoint's warps
-        if (tid == 32 * LZ_EIG_WARPS) S.rr = seq_dot(n, r, r);
-        __syncthreads();
-        if (tid == 0) {
-            S.beta = dd_sqrt(S.rr);
-            S.off[k] = S.beta;
-        }
-        __syncthreads();
         ++k;
         ++kk;
     }
-    if (tid == 0) out[blockIdx.x] = dd_sub(S.mn, dd_abs(dd_mul(S.err, S.beta)));
+    if (rank == 0 && tid == 0) out[cid] = dd_sub(mn, dd_abs(dd_mul(err, beta)));
+}
+
+// CTAs of a block's cluster.  A step's 2 n^2 terms are FP64-bound on one SM
+// from a few dozen rows on and read n^2 dd values of X and n^2 of L through
+// the SMs' L2 ports; four cluster barriers a step cost about 0.2 us each.
+// Whole runs of L L L^T on a B200, us, for 2 / 4 / 8 / 16 CTAs: n = 30: 252 /
+// 258 / 261 / 268; n = 64: 291 / 285 / 291 / 299; n = 100: 406 / 350 / 338 /
+// 343; n = 150: 676 / 518 / 439 / 408; n = 200: 903 / 662 / 520 / 476; n =
+// 500: 3420 / 2207 / 1372 / 990 (one CTA: 6562).  With many blocks the launch
+// fills the GPU by itself.
+int lanczos_cluster(long n, int blocks, int most) {
+    int R = n <= 64 ? 2 : n <= 96 ? 4 : n <= 144 ? 8 : 16;
+    R = std::min(R, most);
+    while (R > 1 && (long)R * blocks > 148) R /= 2;
+    return R;
+}
+
+size_t lanczos_smem(long n, int R, bool vectors) {
+    const long chunks = (n + LZ_CHUNK - 1) / LZ_CHUNK, own = (chunks + R - 1) / R * LZ_CHUNK;
+    return sizeof(LanczosShared) + sizeof(dd_t) * (2 * own + (vectors ? 3 * n : 0));
+}
+
+} // namespace
+
+void launch_lanczos(cudaStream_t st, const int *ids, int nb, int nsp, long maxn, const int *sizes, const long *off, const dd_t *L, const dd_t *D,
+                    const dd_t *L2, const dd_t *D2, dd_t *work, long work_stride, dd_t *out) {
+    constexpr size_t SMEM_MAX = 227 * 1024;
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    // most CTAs a cluster may have here (more than 8 is the device's choice)
+    static thread_local int most[64] = {};
+    if (most[dev & 63] == 0) {
+        for (auto *f : {lanczos_kernel<true>, lanczos_kernel<false>}) {
+            CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+            CK(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        }
+        cudaLaunchConfig_t q = {};
+        q.gridDim = dim3(LZ_CLUSTER);
+        q.blockDim = dim3(LZ_THREADS);
+        q.dynamicSmemBytes = SMEM_MAX;
+        cudaLaunchAttribute a[1];
+        a[0].id = cudaLaunchAttributeClusterDimension;
+        a[0].val.clusterDim.x = LZ_CLUSTER;
+        a[0].val.clusterDim.y = a[0].val.clusterDim.z = 1;
+        q.attrs = a;
+        q.numAttrs = 1;
+        int clusters = 0;
+        const bool ok = cudaOccupancyMaxActiveClusters(&clusters, lanczos_kernel<true>, &q) == cudaSuccess && clusters >= 1;
+        if (!ok) cudaGetLastError();
+        most[dev & 63] = ok ? LZ_CLUSTER : 8;
+    }
+    const int R = lanczos_cluster(maxn, nb * nsp, most[dev & 63]);
+    const bool smem = lanczos_smem(maxn, R, true) <= SMEM_MAX;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nb * nsp * R));
+    cfg.blockDim = dim3(LZ_THREADS);
+    cfg.dynamicSmemBytes = lanczos_smem(maxn, R, smem);
+    cfg.stream = st;
+    cudaLaunchAttribute a[1];
+    a[0].id = cudaLaunchAttributeClusterDimension;
+    a[0].val.clusterDim.x = (unsigned)R;
+    a[0].val.clusterDim.y = a[0].val.clusterDim.z = 1;
+    cfg.attrs = a;
+    cfg.numAttrs = 1;
+    CK(cudaLaunchKernelEx(&cfg, smem ? lanczos_kernel<true> : lanczos_kernel<false>, ids, nb, sizes, off, L, D, L2, D2, work, work_stride, out));
+    CK_LAUNCH();
 }
 
 // Smallest eigenvalue of the lower triangle of an n x n symmetric M
-// (n <= 32): Householder tridiagonalisation, then the warp multisection of
-// tri_min_eigenvalue.  One warp per block: the scalar sums of a reflector
-// on lane 0 in sequence, the products with A and the rank-2 update row by
-// row over the lanes, A in shared memory.
+// (n <= 32): Householder tridiagonalisation, then tri_eig.cuh.  One warp per
+// block, row i on lane i, A in shared memory; the reflectors' sums go over
+// the lanes (a butterfly of five exchanges), the products with A are one
+// compensated dot a lane.  A latency chain of 18 reflections at n = 20: 82 us
+// with the two products that form M; 235 us when lane 0 summed in sequence
+// and a dd Sturm multisection followed.
 __global__ void __launch_bounds__(32) small_min_eig_kernel(const int *blk_ids, const int *sizes, const long *off, const dd_t *Msp, dd_t *out) {
     __shared__ dd_t A[32][33];
-    __shared__ dd_t v[32], p[32], d[32], e[32], e2[32];
-    __shared__ dd_t tau_s, K_s;
-    __shared__ int skip;
+    __shared__ dd_t v[32], w[32], d[32], e[32], ie[32];
+    __shared__ TriWork<32, 1> tri;
     const int lane = threadIdx.x;
     const int b = blk_ids[blockIdx.x];
     const int n = sizes[b];
@@ -411,59 +395,54 @@ __global__ void __launch_bounds__(32) small_min_eig_kernel(const int *blk_ids, c
         }
     __syncwarp();
     for (int k = 0; k + 2 < n; ++k) {
-        if (lane == 0) {
-            skip = 0;
-            dd_t s = dd_zero();
-            for (int i = k + 1; i < n; ++i) s = dd_acc(s, dd_mul(A[i][k], A[i][k]));
-            const dd_t nrm = dd_sqrt(s);
-            if (dd_is_zero(nrm)) {
-                skip = 1;
-            } else {
-                const dd_t alpha = A[k + 1][k].hi < 0.0 ? nrm : dd_neg(nrm);
-                for (int i = 0; i < n; ++i) v[i] = dd_zero();
-                v[k + 1] = dd_sub(A[k + 1][k], alpha);
-                for (int i = k + 2; i < n; ++i) v[i] = A[i][k];
-                dd_t vv = dd_zero();
-                for (int i = k + 1; i < n; ++i) vv = dd_acc(vv, dd_mul(v[i], v[i]));
-                if (dd_is_zero(vv))
-                    skip = 1;
-                else
-                    tau_s = dd_div(dd_from(2.0), vv);
-            }
-        }
+        const bool in = lane > k && lane < n;
+        const dd_t x = in ? A[lane][k] : dd_zero();
+        const dd_t nrm = dd_sqrt(warp_sum_dd(dd_mul(x, x)));
+        if (dd_is_zero(nrm)) continue;
+        // v = x - alpha e_{k+1} with alpha = -sign(x_{k+1}) |x|, and
+        // v.v = 2 |x| (|x| + |x_{k+1}|)
+        const dd_t x1 = A[k + 1][k];
+        const dd_t alpha = x1.hi < 0.0 ? nrm : dd_neg(nrm);
+        const dd_t tau = dd_div(dd_from(1.0), dd_mul(nrm, dd_add(nrm, dd_abs(x1))));
+        const dd_t vi = lane == k + 1 ? dd_sub(x1, alpha) : x;
+        v[lane] = vi;
         __syncwarp();
-        if (skip) continue;
-        const dd_t tau = tau_s;
-        // p = tau A v (row i on lane i)
-        if (lane < n) {
-            dd_t t = dd_zero();
-            for (int j = k + 1; j < n; ++j) t = dd_acc(t, dd_mul(A[lane][j], v[j]));
-            p[lane] = dd_mul(tau, t);
+        // p = tau A v (row i on lane i; row k too: it takes the reflection)
+        dd_t p = dd_zero();
+        if (lane >= k && lane < n) {
+            DotAcc acc;
+            for (int j = k + 1; j < n; ++j) acc.term(make_double2(A[lane][j].hi, A[lane][j].lo), make_double2(v[j].hi, v[j].lo));
+            p = dd_mul(tau, acc.value());
         }
-        __syncwarp();
         // K = tau/2 v^T p ; w = p - K v
-        if (lane == 0) {
-            dd_t vp = dd_zero();
-            for (int i = k + 1; i < n; ++i) vp = dd_acc(vp, dd_mul(v[i], p[i]));
-            K_s = dd_mul(dd_mul_d(tau, 0.5), vp);
-        }
+        const dd_t K = dd_mul(dd_mul_d(tau, 0.5), warp_sum_dd(dd_mul(vi, p)));
+        const dd_t wi = dd_sub(p, dd_mul(K, vi));
+        w[lane] = wi;
         __syncwarp();
-        if (lane < n) p[lane] = dd_sub(p[lane], dd_mul(K_s, v[lane]));
-        __syncwarp();
-        // A -= v w^T + w v^T (row i on lane i)
-        if (lane < n) {
-            const dd_t vi = v[lane], pi = p[lane];
-            for (int j = 0; j < n; ++j) A[lane][j] = dd_sub(dd_sub(A[lane][j], dd_mul(vi, p[j])), dd_mul(pi, v[j]));
+        // A -= v w^T + w v^T on rows and columns k .. n-1 (row i on lane i)
+        if (lane >= k && lane < n) {
+            const double2 nv = make_double2(-vi.hi, -vi.lo), nw = make_double2(-wi.hi, -wi.lo);
+            for (int j = k; j < n; ++j) {
+                DotAcc acc;
+                acc.s = A[lane][j].hi;
+                acc.e = A[lane][j].lo;
+                acc.term(nv, make_double2(w[j].hi, w[j].lo));
+                acc.term(nw, make_double2(v[j].hi, v[j].lo));
+                A[lane][j] = acc.value();
+            }
         }
         __syncwarp();
     }
     if (lane < n) {
         d[lane] = A[lane][lane];
-        if (lane + 1 < n) e[lane] = A[lane + 1][lane];
+        if (lane + 1 < n) {
+            e[lane] = A[lane + 1][lane];
+            ie[lane] = dd_div(dd_from(1.0), e[lane]);
+        }
     }
     __syncwarp();
-    __shared__ unsigned ball[4];
-    const dd_t lam = tri_min_eigenvalue(n, d, e, e2, 1, ball);
+    dd_t lam, last;
+    tri_min_eigenpair<32, 1>(n, d, e, ie, tri, lam, last);
     if (lane == 0) out[blockIdx.x] = lam;
 }
 
@@ -503,11 +482,10 @@ static void min_eig_spaces(Context &c, int nsp, const Space *L[2], const Space *
     if (nb > 0) {
         long maxn = 0;
         for (int l : big) maxn = std::max<long>(maxn, c.sizes[l]);
-        c.eig_work.alloc(5 * maxn * nb * nsp);
-        // the two spaces' CTAs write slots 0 .. 2 nb - 1; spread below
-        lanczos_kernel<<<(unsigned)(nb * nsp), LZ_THREADS, 0, st>>>(c.eig_ids_big.p, (int)nb, c.d_sizes.p, c.d_off.p, L[0]->buf.p, D[0]->buf.p,
-                                                                   L[nsp - 1]->buf.p, D[nsp - 1]->buf.p, c.eig_work.p, 5 * maxn, res + 2 * c.nSDP);
-        CK_LAUNCH();
+        c.eig_work.alloc(LZ_WORK * maxn * nb * nsp);
+        // the two spaces' clusters write slots 0 .. 2 nb - 1; spread below
+        launch_lanczos(st, c.eig_ids_big.p, (int)nb, nsp, maxn, c.d_sizes.p, c.d_off.p, L[0]->buf.p, D[0]->buf.p, L[nsp - 1]->buf.p,
+                       D[nsp - 1]->buf.p, c.eig_work.p, LZ_WORK * maxn, res + 2 * c.nSDP);
     }
     for (int sp = 0; sp < nsp && ns > 0; ++sp) small_blocks(c, *L[sp], *D[sp], small, res + (size_t)sp * c.nSDP + nb);
     if (nb > 0) {

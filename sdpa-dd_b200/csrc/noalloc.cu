@@ -36,11 +36,12 @@ constexpr long NOALLOC_MAX_N = SDDD_MIN_EIG_NOALLOC_MAX_N;
 // Order up to which the block takes the dense path (two GEMMs and a
 // tridiagonal eigenvalue), as Jal::getMinEigen (sdpa_jordan.cpp:55-88).
 constexpr long SMALL_N = 20;
-// Header (block id, order, offset) in the first 256 bytes, then five Lanczos
-// vectors of the largest order; the dense path's two n x n products fit in
+// Header (block id, order, offset) in the first 256 bytes, then room for the Lanczos
+// vectors (LZ_WORK of the largest order); the dense path's two n x n products fit in
 // the same region.
 constexpr long HEADER_DD = 16;
 constexpr long NOALLOC_SCRATCH_DD = HEADER_DD + 5 * NOALLOC_MAX_N;
+static_assert(LZ_WORK <= 5, "Lanczos vectors fit their region");
 static_assert(2 * SMALL_N * SMALL_N <= 5 * NOALLOC_MAX_N, "dense path fits the Lanczos region");
 
 static __device__ __align__(256) double2 g_noalloc_scratch[NOALLOC_SCRATCH_DD];
@@ -117,8 +118,7 @@ extern "C" int sddd_min_eig_noalloc(void *stream, long n, const sddd_dd *L, cons
         noalloc_header_kernel<<<1, 1, 0, st>>>(ids, sizes, off, (int)n);
         CK_LAUNCH();
         if (n > SMALL_N) {
-            lanczos_kernel<<<1, LZ_THREADS, 0, st>>>(ids, 1, sizes, off, Ld, Dd, Ld, Dd, work, 5 * n, o);
-            CK_LAUNCH();
+            launch_lanczos(st, ids, 1, 1, n, sizes, off, Ld, Dd, Ld, Dd, work, LZ_WORK * n, o);
         } else {
             // W2 = D L^T (Rgemm "N","T"), W1 = L W2 (Rgemm "N","N")
             const int m = (int)n;
