@@ -19,6 +19,7 @@
 // reorders the operations that land on one entry.
 #include "blas.h"
 #include "bulk.cuh"
+#include "devops.cuh"
 #include "ozaki.h"
 #include "prof.h"
 
@@ -1091,22 +1092,20 @@ void axpy(cudaStream_t st, const dd_t *x, const dd_t *y, dd_t *z, long n, dd_t a
 constexpr int DOT_SEQ = 1024;
 constexpr int DOT_THREADS = 256;
 
-__global__ void dot_seq_kernel(const dd_t *x, long incx, const dd_t *y, long incy, long n, dd_t *out) {
-    if (threadIdx.x != 0) return;
-    dd_t t = dd_zero();
-    for (long i = 0; i < n; ++i) t = dd_acc(t, dd_mul(ld_dd(x + i * incx), ld_dd(y + i * incy)));
-    st_dd(out, dd_acc(dd_zero(), t));
+__global__ void __launch_bounds__(CHAIN_THREADS) dot_seq_kernel(const dd_t *x, long incx, const dd_t *y, long incy, long n, dd_t *out) {
+    __shared__ double2 buf[2][CHAIN_CHUNK];
+    const dd_t t = cta_chain(n, [&](long i) { return dd_mul(ld_dd(x + i * incx), ld_dd(y + i * incy)); }, buf);
+    if (threadIdx.x == 0) st_dd(out, dd_acc(dd_zero(), t));
 }
 
 // Chains of a batch of equal-length dot products: CTA b, x + b sx, y + b
 // sy, result out[b].
-__global__ void dot_seq_batch_kernel(const dd_t *x, long sx, const dd_t *y, long sy, long n, dd_t *out) {
-    if (threadIdx.x != 0) return;
+__global__ void __launch_bounds__(CHAIN_THREADS) dot_seq_batch_kernel(const dd_t *x, long sx, const dd_t *y, long sy, long n, dd_t *out) {
+    __shared__ double2 buf[2][CHAIN_CHUNK];
     x += blockIdx.x * sx;
     y += blockIdx.x * sy;
-    dd_t t = dd_zero();
-    for (long i = 0; i < n; ++i) t = dd_acc(t, dd_mul(ld_dd(x + i), ld_dd(y + i)));
-    st_dd(out + blockIdx.x, dd_acc(dd_zero(), t));
+    const dd_t t = cta_chain(n, [&](long i) { return dd_mul(ld_dd(x + i), ld_dd(y + i)); }, buf);
+    if (threadIdx.x == 0) st_dd(out + blockIdx.x, dd_acc(dd_zero(), t));
 }
 
 __device__ dd_t block_tree(dd_t v, double2 *sh) {
@@ -1144,7 +1143,7 @@ __global__ void tree_final_kernel(const dd_t *partial, int np, dd_t *out) {
 
 void dot(cudaStream_t st, const dd_t *x, long incx, const dd_t *y, long incy, long n, dd_t *out, dd_t *scratch) {
     if (n <= DOT_SEQ) {
-        dot_seq_kernel<<<1, 32, 0, st>>>(x, incx, y, incy, n, out);
+        dot_seq_kernel<<<1, CHAIN_THREADS, 0, st>>>(x, incx, y, incy, n, out);
         CK_LAUNCH();
         return;
     }
@@ -1158,7 +1157,7 @@ void dot(cudaStream_t st, const dd_t *x, long incx, const dd_t *y, long incy, lo
 void dot_batched(cudaStream_t st, const dd_t *x, long sx, const dd_t *y, long sy, long n, int batch, dd_t *out, dd_t *scratch) {
     if (batch <= 0) return;
     if (n <= DOT_SEQ) {
-        dot_seq_batch_kernel<<<batch, 32, 0, st>>>(x, sx, y, sy, n, out);
+        dot_seq_batch_kernel<<<batch, CHAIN_THREADS, 0, st>>>(x, sx, y, sy, n, out);
         CK_LAUNCH();
         return;
     }
@@ -1183,16 +1182,22 @@ __global__ void maxabs_kernel(const dd_t *x, long n, dd_t *partial) {
     if (threadIdx.x == 0) partial[blockIdx.x] = dd_make(sh[0].x, sh[0].y);
 }
 __global__ void max_final_kernel(const dd_t *partial, int np, dd_t *out) {
+    __shared__ double2 sh[DOT_THREADS];
+    if (threadIdx.x < np) {
+        const dd_t v = ld_dd(partial + threadIdx.x);
+        sh[threadIdx.x] = make_double2(v.hi, v.lo);
+    }
+    __syncthreads();
     if (threadIdx.x != 0) return;
     dd_t m = dd_zero();
-    for (int i = 0; i < np; ++i) m = dd_max(m, partial[i]);
+    for (int i = 0; i < np; ++i) m = dd_max(m, dd_make(sh[i].x, sh[i].y));
     *out = m;
 }
 void maxabs(cudaStream_t st, const dd_t *x, long n, dd_t *out, dd_t *scratch) {
     int nb = (int)std::min<long>(DOT_THREADS, std::max(1u, ceil_div(n, 4L * DOT_THREADS)));
     maxabs_kernel<<<nb, DOT_THREADS, 0, st>>>(x, n, scratch);
     CK_LAUNCH();
-    max_final_kernel<<<1, 32, 0, st>>>(scratch, nb, out);
+    max_final_kernel<<<1, DOT_THREADS, 0, st>>>(scratch, nb, out);
     CK_LAUNCH();
 }
 

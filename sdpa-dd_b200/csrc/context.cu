@@ -417,6 +417,9 @@ void upload_problem(Context &c, Problem &&p) {
     c.views.upload(views, c.stream);
     c.d_off.upload(c.off, c.stream);
     c.d_sizes.upload(c.sizes, c.stream);
+    std::vector<int> dim(c.nSDP + 1, 0);
+    for (int l = 0; l < c.nSDP; ++l) dim[l + 1] = dim[l] + c.sizes[l];
+    c.d_dim.upload(dim, c.stream);
     std::vector<int> ptr(c.m + 1, 0), bl, tt;
     for (int k = 0; k < c.m; ++k) {
         for (auto &kv : P.A[k]) {

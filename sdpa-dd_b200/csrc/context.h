@@ -189,6 +189,7 @@ struct Context {
     DBuf<BlockView> views; // [l]
     DBuf<long> d_off;      // [l] block offsets within a space
     DBuf<int> d_sizes;     // [l] block sizes
+    DBuf<int> d_dim;       // [l] rows before block l; [nSDP] all rows
     // per constraint: (block, t) pairs ascending by block
     DBuf<int> cb_ptr, cb_block, cb_t;
     // every constraint is one dense matrix of the single SDP block, whose

@@ -382,29 +382,29 @@ int ScalarBatch::inner_space(const Space &a, const Space &b) {
     return g;
 }
 
-__global__ void sparse_inner_kernel(int n, int nnz, const int *row, const int *col, const dd_t *val, const dd_t *D, dd_t *out) {
-    if (threadIdx.x == 0) st_dd(out, sparse_dot_dense(n, nnz, row, col, val, D));
-}
-
 // The blocks whose product with C is one chain (sparse C, or dense C of at
 // most DOT_SEQ_TERMS entries) in one launch: CTA l, result to its slot.
 constexpr long DOT_SEQ_TERMS = 1024; // the longest dot that dot() runs as one chain
-__global__ void inner_C_small_kernel(const BlockView *views, const int *slot, const long *off, const dd_t *x, dd_t *out) {
-    if (threadIdx.x != 0) return;
+__global__ void __launch_bounds__(CHAIN_THREADS) inner_C_small_kernel(const BlockView *views, const int *slot, const long *off, const dd_t *x,
+                                                                    dd_t *out) {
+    __shared__ double2 buf[2][CHAIN_CHUNK];
     const int l = blockIdx.x;
-    const BlockView v = views[l];
+    const BlockView &v = views[l];
     const int s = slot[l];
     if (s < 0 || !v.c_present) return;
     const dd_t *D = x + off[l];
+    dd_t r;
     if (!v.c_dense) {
-        st_dd(out + s, sparse_dot_dense(v.n, v.c_nnz, v.c_row, v.c_col, v.c_val, D));
-        return;
+        const int n = v.n, nnz = v.c_nnz, *row = v.c_row, *col = v.c_col;
+        const dd_t *val = v.c_val;
+        r = cta_chain(sparse_dot_steps(nnz), [&](long e) { return sparse_dot_step(n, nnz, row, col, val, D, (int)e); }, buf);
+    } else {
+        const long nn = (long)v.n * v.n;
+        if (nn > DOT_SEQ_TERMS) return;
+        const dd_t *C = v.c_dense_val;
+        r = dd_acc(dd_zero(), cta_chain(nn, [&](long e) { return dd_mul(ld_dd(C + e), ld_dd(D + e)); }, buf));
     }
-    const long nn = (long)v.n * v.n;
-    if (nn > DOT_SEQ_TERMS) return;
-    dd_t t = dd_zero();
-    for (long i = 0; i < nn; ++i) t = dd_acc(t, dd_mul(ld_dd(v.c_dense_val + i), ld_dd(D + i)));
-    st_dd(out + s, dd_acc(dd_zero(), t));
+    if (threadIdx.x == 0) st_dd(out + s, r);
 }
 
 // Lal::getInnerProduct(SparseLinearSpace C, DenseLinearSpace X)
@@ -421,7 +421,7 @@ int ScalarBatch::inner_C(const Space &x) {
     const int g = group(c.c_nslots);
     if (c.c_nslots == 0) return g;
     dd_t *out = c.scal.p + groups[g].first;
-    inner_C_small_kernel<<<c.nSDP, 32, 0, c.stream>>>(c.views.p, c.c_slot.p, c.d_off.p, x.buf.p, out);
+    inner_C_small_kernel<<<c.nSDP, CHAIN_THREADS, 0, c.stream>>>(c.views.p, c.c_slot.p, c.d_off.p, x.buf.p, out);
     CK_LAUNCH();
     for (int l = 0; l < c.nSDP; ++l) {
         const BlockDev &bd = *c.blocks[l];
@@ -493,19 +493,30 @@ void residuals(Context &c, dd_t &normPrimal, dd_t &normDual) {
     normDual = sb.value(gd);
 }
 
-__global__ void lambda_trace_kernel(const dd_t *S, const long *off, const int *sizes, int nb, double lambda, dd_t *out) {
-    if (threadIdx.x != 0) return;
-    dd_t r = dd_zero();
-    for (int b = 0; b < nb; ++b) {
-        const int n = sizes[b];
-        for (int i = 0; i < n; ++i) r = dd_acc(r, dd_mul_d(ld_dd(S + off[b] + i + (long)n * i), lambda));
-    }
-    st_dd(out, r);
+// sum_b sum_i S_b(i,i) lambda in order; dim[b]: rows before block b.
+__global__ void __launch_bounds__(CHAIN_THREADS) lambda_trace_kernel(const dd_t *S, const long *off, const int *dim, int nb, double lambda, dd_t *out) {
+    __shared__ double2 buf[2][CHAIN_CHUNK];
+    const dd_t r = cta_chain(
+        dim[nb],
+        [&](long e) {
+            int lo = 0, hi = nb; // the block with dim[lo] <= e < dim[lo + 1]
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) / 2;
+                if (dim[mid] <= e)
+                    lo = mid;
+                else
+                    hi = mid;
+            }
+            const long i = e - dim[lo], n = dim[lo + 1] - dim[lo];
+            return dd_mul_d(ld_dd(S + off[lo] + i + n * i), lambda);
+        },
+        buf);
+    if (threadIdx.x == 0) st_dd(out, r);
 }
 
 int ScalarBatch::lambda_trace(const Space &s, double lambda) {
     const int g = group(1);
-    lambda_trace_kernel<<<1, 32, 0, c.stream>>>(s.buf.p, c.d_off.p, c.d_sizes.p, c.nSDP, lambda, c.scal.p + groups[g].first);
+    lambda_trace_kernel<<<1, CHAIN_THREADS, 0, c.stream>>>(s.buf.p, c.d_off.p, c.d_dim.p, c.nSDP, lambda, c.scal.p + groups[g].first);
     CK_LAUNCH();
     return g;
 }
