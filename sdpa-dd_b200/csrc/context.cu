@@ -431,8 +431,42 @@ void upload_problem(Context &c, Problem &&p) {
         }
         ptr[k + 1] = (int)bl.size();
     }
-    c.inner_dense1 = c.nSDP == 1 && c.m > 0 && (int)bl.size() == c.m && c.blocks[0]->all_dense &&
-                     (size_t)c.sizes[0] * c.sizes[0] * sizeof(dd_t) <= INNER_DENSE1_SMEM;
+    {
+        std::vector<std::vector<int>> dense(c.nSDP); // positions by block
+        std::vector<InnerTask> tasks;
+        std::vector<int> it, at;
+        std::vector<std::pair<int, int>> sparse; // (-steps, position)
+        for (int p = 0; p < (int)bl.size(); ++p) {
+            const BlockMat &M = P.A[P.cons[bl[p]][tt[p]]].at(bl[p]);
+            const int nnz = (int)M.row.size(), steps = nnz / 4 + nnz % 4;
+            if (M.dense)
+                dense[bl[p]].push_back(p);
+            else if (steps >= INNER_LONG)
+                sparse.push_back({-steps, p});
+        }
+        std::sort(sparse.begin(), sparse.end());
+        if (sparse.size() > INNER_SPARSE) sparse.resize(INNER_SPARSE);
+        for (auto &sp : sparse) {
+            tasks.push_back({bl[sp.second], (int)it.size(), -1});
+            it.push_back(tt[sp.second]);
+            at.push_back(sp.second);
+        }
+        for (int l = 0; l < c.nSDP; ++l)
+            for (size_t q = 0; q < dense[l].size(); ++q) {
+                if (q % 32 == 0) tasks.push_back({l, (int)it.size(), 0});
+                ++tasks.back().count;
+                it.push_back(tt[dense[l][q]]);
+                at.push_back(dense[l][q]);
+            }
+        // long sums first
+        std::stable_sort(tasks.begin(), tasks.end(), [&](const InnerTask &a, const InnerTask &b) { return c.sizes[a.block] > c.sizes[b.block]; });
+        c.n_inner_tasks = (int)tasks.size();
+        c.inner_tasks.upload(tasks, c.stream);
+        c.inner_t.upload(it, c.stream);
+        c.inner_at.upload(at, c.stream);
+        if (!tasks.empty()) c.inner_prod.alloc(bl.size());
+        for (int p : at) tt[p] = -1;
+    }
     c.cb_ptr.upload(ptr, c.stream);
     c.cb_block.upload(bl, c.stream);
     c.cb_t.upload(tt, c.stream);

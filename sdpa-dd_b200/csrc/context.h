@@ -48,11 +48,19 @@ struct DBuf {
     }
 };
 
-// Kernel-side view of one block's problem data (pointers into BlockDev).
-// Largest single block (bytes of n x n dd) whose constraint inner products
-// take the shared-memory form (constraint_inner).
-constexpr size_t INNER_DENSE1_SMEM = 160 * 1024;
+// Products A . M of the constraints' matrices with one block that one warp
+// forms (constraint_inner): `count` dense matrices, or, with count = -1, one
+// sparse matrix: the INNER_SPARSE longest sums of at least INNER_LONG steps
+// (the others are formed by their constraint's thread, all side by side,
+// where a step is a chain of two memory latencies, about 1 us; a task's
+// launch and hand-over take about 6 us, and more tasks than the GPU holds at
+// once would run one after the other).
+constexpr int INNER_LONG = 8, INNER_SPARSE = 256;
+struct InnerTask {
+    int block, first, count;
+};
 
+// Kernel-side view of one block's problem data (pointers into BlockDev).
 struct BlockView {
     int n, nc, nsparse, all_dense;
     const int *con, *formula, *perm, *coo_off, *nnz;
@@ -191,10 +199,14 @@ struct Context {
     DBuf<int> d_sizes;     // [l] block sizes
     DBuf<int> d_dim;       // [l] rows before block l; [nSDP] all rows
     // per constraint: (block, t) pairs ascending by block
+    // (t = -1: the product is formed by a task, below)
     DBuf<int> cb_ptr, cb_block, cb_t;
-    // every constraint is one dense matrix of the single SDP block, whose
-    // order fits the shared-memory form of the constraint inner products
-    bool inner_dense1 = false;
+    // the tasks of constraint_inner, their matrices (t in the block, position
+    // in cb_*), grouped by block, and the products by position
+    DBuf<InnerTask> inner_tasks;
+    DBuf<int> inner_t, inner_at;
+    DBuf<dd_t> inner_prod;
+    int n_inner_tasks = 0;
     DBuf<dd_t> b;
     // iterate and derived (Solutions)
     Space X, Z, invCholX, invCholZ, invZ;

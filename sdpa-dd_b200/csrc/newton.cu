@@ -17,90 +17,154 @@ static const dd_t MONE = {-1.0, 0.0};
 // --------------------------------------------------- per-constraint A_k . M
 // InputData::multi_InnerProductToA (sdpa_dataset.cpp:477-485) followed by
 // "v = v * (-1); v = v + w" (the callers' Lal::let pair, Rscal then Raxpy).
+//
+// The product of a dense constraint matrix with a block of M is one chain of
+// n^2 dd sums (Rdot's order), so a kernel can do no better than that chain's
+// latency, 8 dependent FP64 operations (63 cycles) a term, and has to keep
+// everything else off it.  inner_pairs_kernel gives a CTA up to 32 matrices
+// of one block, one a lane of warp 0, which only adds: warp 1 brings the
+// chunk of 32 terms of every matrix after next (cp.async, 512 contiguous
+// bytes an instruction), warps 2 and 3 form the products of the next chunk
+// (a term at a lane; rows are 33 entries apart, so that warp 0 reads them
+// without bank conflicts).  Sparse matrices with long sums go through it
+// too, one a CTA, the terms formed by all threads.  Then one thread a
+// constraint adds its blocks' products in block order, short sparse products
+// formed on the spot.
+// Blocks 100 + 50, m = 1326: 0.40 ms; with the products formed by the adding
+// warp 0.49 ms (the multiplications delay the chain in the FP64 pipe); one
+// thread a constraint that streamed its matrices from global memory, block
+// after block, took 2.24 ms.
+constexpr int IP_CHUNK = 32, IP_LD = IP_CHUNK + 1, IP_THREADS = 128;
+constexpr size_t IP_SMEM = sizeof(double2) * (4 * 32 * IP_LD + 2 * IP_CHUNK); // raw and product stages, M
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__global__ void __launch_bounds__(IP_THREADS) inner_pairs_kernel(const InnerTask *tasks, const int *pair_t, const int *pair_at,
+                                                                const BlockView *views, const long *off, const dd_t *M, dd_t *prod) {
+    extern __shared__ double2 ip_sm[];
+    const InnerTask task = tasks[blockIdx.x];
+    const BlockView &v = views[task.block];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = v.n;
+    const dd_t *Ml = M + off[task.block];
+    if (task.count < 0) {
+        // one sparse matrix
+        const int t = pair_t[task.first], o = v.coo_off[t], nnz = v.nnz[t], steps = sparse_dot_steps(nnz);
+        const int *row = v.row + o, *col = v.col + o;
+        const dd_t *val = v.val + o;
+        constexpr int BUF = 4 * 32 * IP_LD;
+        dd_t r = dd_zero();
+        for (int base = 0; base < steps; base += BUF) {
+            const int len = min(BUF, steps - base);
+            for (int e = tid; e < len; e += IP_THREADS) {
+                const dd_t x = sparse_dot_step(n, nnz, row, col, val, Ml, base + e);
+                ip_sm[e] = make_double2(x.hi, x.lo);
+            }
+            __syncthreads();
+            if (tid == 0)
+                for (int e = 0; e < len; ++e) r = dd_acc(r, dd_make(ip_sm[e].x, ip_sm[e].y));
+            __syncthreads();
+        }
+        if (tid == 0) st_dd(prod + pair_at[task.first], r);
+        return;
+    }
+    const long nn = (long)n * n;
+    const dd_t *A = v.dense + v.dense_off[pair_t[task.first + min(lane, task.count - 1)]];
+    double2 *raw = ip_sm, *prd = ip_sm + 2 * 32 * IP_LD, *Ms = ip_sm + 4 * 32 * IP_LD;
+    auto load = [&](long k0, int stage) { // warp 1
+        if (k0 + lane < nn) cp_async16(Ms + stage * IP_CHUNK + lane, Ml + k0 + lane);
+        for (int r = 0; r < task.count; ++r) {
+            const dd_t *row = reinterpret_cast<const dd_t *>(__shfl_sync(0xffffffffu, (unsigned long long)A, r));
+            if (k0 + lane < nn) cp_async16(raw + (stage * 32 + r) * IP_LD + lane, row + k0 + lane);
+        }
+        cp_async_commit();
+    };
+    auto form = [&](int stage) { // warps 2 and 3; terms past nn are never added
+        const double2 y = Ms[stage * IP_CHUNK + lane];
+        for (int r = warp - 2; r < task.count; r += 2) {
+            const int at = (stage * 32 + r) * IP_LD + lane;
+            const double2 x = raw[at];
+            const dd_t q = dd_mul(dd_make(x.x, x.y), dd_make(y.x, y.y));
+            prd[at] = make_double2(q.hi, q.lo);
+        }
+    };
+    if (warp == 1) {
+        load(0, 0);
+        cp_async_wait<0>();
+    }
+    __syncthreads();
+    if (warp == 1 && IP_CHUNK < nn) load(IP_CHUNK, 1);
+    if (warp >= 2) form(0);
+    dd_t t = dd_zero();
+    int stage = 0;
+    for (long k0 = 0; k0 < nn; k0 += IP_CHUNK, stage ^= 1) {
+        if (warp == 1) cp_async_wait<0>();
+        __syncthreads();
+        if (warp > 0) {
+            // chunk k0's products are formed; its raw stage is free
+            if (warp == 1 && k0 + 2 * IP_CHUNK < nn) load(k0 + 2 * IP_CHUNK, stage);
+            if (warp >= 2 && k0 + IP_CHUNK < nn) form(stage ^ 1);
+            continue;
+        }
+        const double2 *p = prd + (stage * 32 + min(lane, task.count - 1)) * IP_LD;
+        if (nn - k0 >= IP_CHUNK) {
+            double2 x[2][8]; // the next eight come while these are added
+#pragma unroll
+            for (int u = 0; u < 8; ++u) x[0][u] = p[u];
+#pragma unroll
+            for (int q = 0; q < IP_CHUNK / 8; ++q) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (q + 1 < IP_CHUNK / 8) x[(q + 1) & 1][u] = p[8 * (q + 1) + u];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) t = dd_acc(t, dd_make(x[q & 1][u].x, x[q & 1][u].y));
+            }
+        } else {
+            const int len = (int)(nn - k0);
+            for (int k = 0; k < len; ++k) t = dd_acc(t, dd_make(p[k].x, p[k].y));
+        }
+    }
+    if (warp == 0 && lane < task.count) st_dd(prod + pair_at[task.first + lane], dd_acc(dd_zero(), t));
+}
+
 __global__ void constraint_inner_kernel(int m, const BlockView *views, const long *off, const int *cb_ptr, const int *cb_block, const int *cb_t,
-                                        const dd_t *M, const dd_t *addv, dd_t *out) {
+                                        const dd_t *M, const dd_t *prod, const dd_t *addv, dd_t *out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     dd_t ret = dd_zero();
     for (int p = cb_ptr[i]; p < cb_ptr[i + 1]; ++p) {
-        const int l = cb_block[p], t = cb_t[p];
-        const BlockView &v = views[l];
-        const dd_t *Ml = M + off[l];
+        const int l = cb_block[p], t = cb_t[p]; // t < 0: formed by a task
         dd_t tmp;
-        const long doff = v.dense_off[t];
-        if (doff >= 0) {
-            tmp = seq_dot((long)v.n * v.n, v.dense + doff, Ml);
+        if (t < 0) {
+            tmp = ld_dd(prod + p);
         } else {
+            const BlockView &v = views[l];
             const int o = v.coo_off[t];
-            tmp = sparse_dot_dense(v.n, v.nnz[t], v.row + o, v.col + o, v.val + o, Ml);
+            tmp = sparse_dot_dense(v.n, v.nnz[t], v.row + o, v.col + o, v.val + o, M + off[l]);
         }
         ret = dd_acc(ret, tmp);
     }
     st_dd(out + i, dd_acc(dd_mul(MONE, ret), dd_mul(ONE, ld_dd(addv + i))));
 }
 
-// The same for one SDP block whose constraints are all dense: the block of
-// M is staged in shared memory once per CTA (every thread reads the same
-// entry at the same step), and each thread streams its constraint's n^2
-// entries with the next 16 in flight while it sums the current 16, in
-// Rdot's order.
-constexpr int INNER_CHUNK = 16;
-constexpr int INNER_DENSE1_THREADS = 128;
-__global__ void __launch_bounds__(INNER_DENSE1_THREADS) constraint_inner_dense1_kernel(int m, const BlockView *views, const int *cb_ptr,
-                                                                                     const int *cb_t, const dd_t *M, const dd_t *addv, dd_t *out) {
-    extern __shared__ double2 ms[];
-    const int n = views[0].n;
-    const long nn = (long)n * n;
-    for (long e = threadIdx.x; e < nn; e += blockDim.x) ms[e] = *reinterpret_cast<const double2 *>(M + e);
-    __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const dd_t *A = views[0].dense + views[0].dense_off[cb_t[cb_ptr[i]]];
-    dd_t t = dd_zero();
-    dd_t a[INNER_CHUNK], b[INNER_CHUNK];
-    const long full = nn / INNER_CHUNK * INNER_CHUNK;
-    if (full > 0) {
-#pragma unroll
-        for (int u = 0; u < INNER_CHUNK; ++u) a[u] = ld_dd(A + u);
-    }
-    for (long k = 0; k < full; k += INNER_CHUNK) {
-#pragma unroll
-        for (int u = 0; u < INNER_CHUNK; ++u) b[u] = a[u];
-        if (k + INNER_CHUNK < full) {
-#pragma unroll
-            for (int u = 0; u < INNER_CHUNK; ++u) a[u] = ld_dd(A + k + INNER_CHUNK + u);
-        }
-#pragma unroll
-        for (int u = 0; u < INNER_CHUNK; ++u) {
-            const double2 y = ms[k + u];
-            t = dd_acc(t, dd_mul(b[u], dd_make(y.x, y.y)));
-        }
-    }
-    for (long k = full; k < nn; ++k) {
-        const double2 y = ms[k];
-        t = dd_acc(t, dd_mul(ld_dd(A + k), dd_make(y.x, y.y)));
-    }
-    // seq_dot's "0 + templ", then the caller's ret += tmp from zero
-    const dd_t ret = dd_acc(dd_zero(), dd_acc(dd_zero(), t));
-    st_dd(out + i, dd_acc(dd_mul(MONE, ret), dd_mul(ONE, ld_dd(addv + i))));
-}
-
 void constraint_inner(Context &c, const Space &M, const dd_t *addv, dd_t *out) {
-    if (c.inner_dense1) {
-        const size_t smem = sizeof(dd_t) * (size_t)c.sizes[0] * c.sizes[0];
+    if (c.n_inner_tasks > 0) {
         static thread_local bool attr[64] = {};
         int dev = 0;
         CK(cudaGetDevice(&dev));
         if (!attr[dev & 63]) {
-            CK(cudaFuncSetAttribute(constraint_inner_dense1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INNER_DENSE1_SMEM));
+            CK(cudaFuncSetAttribute(inner_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IP_SMEM));
             attr[dev & 63] = true;
         }
-        constraint_inner_dense1_kernel<<<ceil_div(c.m, INNER_DENSE1_THREADS), INNER_DENSE1_THREADS, smem, c.stream>>>(
-            c.m, c.views.p, c.cb_ptr.p, c.cb_t.p, M.buf.p + c.off[0], addv, out);
+        inner_pairs_kernel<<<c.n_inner_tasks, IP_THREADS, IP_SMEM, c.stream>>>(c.inner_tasks.p, c.inner_t.p, c.inner_at.p, c.views.p, c.d_off.p, M.buf.p,
+                                                                      c.inner_prod.p);
         CK_LAUNCH();
-        return;
     }
-    constraint_inner_kernel<<<ceil_div(c.m, 64), 64, 0, c.stream>>>(c.m, c.views.p, c.d_off.p, c.cb_ptr.p, c.cb_block.p, c.cb_t.p, M.buf.p, addv, out);
+    constraint_inner_kernel<<<ceil_div(c.m, 64), 64, 0, c.stream>>>(c.m, c.views.p, c.d_off.p, c.cb_ptr.p, c.cb_block.p, c.cb_t.p, M.buf.p,
+                                                                    c.inner_prod.p, addv, out);
     CK_LAUNCH();
 }
 
