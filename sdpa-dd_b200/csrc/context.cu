@@ -467,6 +467,17 @@ void upload_problem(Context &c, Problem &&p) {
         if (!tasks.empty()) c.inner_prod.alloc(bl.size());
         for (int p : at) tt[p] = -1;
     }
+    {
+        // long chains first
+        std::vector<int> order(c.nSDP);
+        std::iota(order.begin(), order.end(), 0);
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return c.blocks[a]->nc > c.blocks[b]->nc; });
+        std::vector<int2> tasks;
+        for (int l : order)
+            for (long e = 0; e < (long)c.sizes[l] * c.sizes[l]; e += 128) tasks.push_back(make_int2(l, (int)(e / 128)));
+        c.n_yA_tasks = (int)tasks.size();
+        c.yA_tasks.upload(tasks, c.stream);
+    }
     c.cb_ptr.upload(ptr, c.stream);
     c.cb_block.upload(bl, c.stream);
     c.cb_t.upload(tt, c.stream);

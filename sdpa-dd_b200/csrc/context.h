@@ -207,6 +207,9 @@ struct Context {
     DBuf<int> inner_t, inner_at;
     DBuf<dd_t> inner_prod;
     int n_inner_tasks = 0;
+    // (block, 128-entry chunk) of each CTA of sum_k y_k A_k
+    DBuf<int2> yA_tasks;
+    int n_yA_tasks = 0;
     DBuf<dd_t> b;
     // iterate and derived (Solutions)
     Space X, Z, invCholX, invCholZ, invZ;

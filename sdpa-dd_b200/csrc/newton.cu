@@ -172,44 +172,74 @@ void constraint_inner(Context &c, const Space &M, const dd_t *addv, dd_t *out) {
 // InputData::multi_plusToA (sdpa_dataset.cpp:488-493), entry by entry, then
 // mode 0 (compute_DzMat, sdpa_newton.cpp:1318-1327): r = -r (+ D)
 // mode 1 (Residuals::compute, sdpa_dataset.cpp:632-636): r = -r + C - Z
-// One launch per run of equal blocks: CTA row t takes block first + t.
-__global__ void sum_yA_kernel(const BlockView *views, int first, long nn, const dd_t *y, dd_t *out, int mode, const dd_t *D, const dd_t *Z) {
-    const BlockView v = views[first + blockIdx.y];
-    const long ne = (long)v.n * v.n;
-    const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (e >= ne) return;
-    out += blockIdx.y * nn;
-    if (D) D += blockIdx.y * nn;
-    if (Z) Z += blockIdx.y * nn;
+// One launch: CTA b takes the 128 entries of tasks[b] = (block, 128-chunk).
+//
+// Where every matrix of the block is dense, an entry's sum is a chain of dd
+// multiply-adds over the constraints at 16 n^2 bytes a step, so a thread
+// needs more loads in flight than the compiler keeps in registers: its terms
+// come through a ring in shared memory, two stages of twelve terms, each
+// thread copying and waiting for its own (cp.async), the y_k through a small
+// ring a warp.  Bound by the chain, about 165 cycles a term with the product
+// in it.  Blocks 100 + 50, m = 1326: 126 us; with eight loads ahead in
+// registers and a launch a block 920 us; with the products formed by other
+// warps, from registers, 180 us.  Stages of 8 terms, two or three: 145 us; of
+// 16: 123 us, but slower where a block has few constraints.
+constexpr int YA_THREADS = 128, YA_TERMS = 12, YA_STAGES = 2;
+constexpr size_t YA_SMEM = sizeof(double2) * YA_STAGES * YA_TERMS * (YA_THREADS + YA_THREADS / 32);
+static_assert(YA_TERMS <= 32, "a lane a y_k");
+__global__ void __launch_bounds__(YA_THREADS) sum_yA_kernel(const BlockView *views, const int2 *tasks, const long *off, const dd_t *y, dd_t *out,
+                                                           int mode, const dd_t *D, const dd_t *Z) {
+    extern __shared__ double2 ya_sm[];
+    const int2 task = tasks[blockIdx.x];
+    const BlockView &v = views[task.x];
+    const long ne = (long)v.n * v.n, base = off[task.x];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const long e = (long)task.y * YA_THREADS + tid;
     dd_t acc = dd_zero();
     if (v.all_dense) {
-        // the operands of eight steps go out ahead of their terms (the
-        // sum's order is unchanged)
-        int t = 0;
-        for (; t + 8 <= v.nc; t += 8) {
-            long o[8];
-            int k[8];
+        constexpr int RING = YA_STAGES * YA_TERMS;
+        double2 *ring = ya_sm + tid, *yr = ya_sm + RING * YA_THREADS + (tid >> 5) * RING;
+        const dd_t *A = v.dense + (e < ne ? e : ne - 1); // matrix t at t n^2
+        const int *con = v.con, nc = v.nc;
+        int k = lane < YA_TERMS && lane < nc ? con[lane] : 0; // of the next stage to go out
+        auto issue = [&](int s) {
+            const int t0 = s * YA_TERMS, slot = s % YA_STAGES * YA_TERMS;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                o[u] = v.dense_off[t + u];
-                k[u] = v.con[t + u];
+            for (int u = 0; u < YA_TERMS; ++u)
+                if (t0 + u < nc) cp_async16(ring + (slot + u) * YA_THREADS, A + (t0 + u) * ne);
+            if (lane < YA_TERMS && t0 + lane < nc) {
+                cp_async16(yr + slot + lane, y + k);
+                if (t0 + YA_TERMS + lane < nc) k = con[t0 + YA_TERMS + lane];
             }
-            dd_t a[8], b[8];
+            cp_async_commit();
+        };
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                a[u] = ld_dd(v.dense + o[u] + e);
-                b[u] = ld_dd(y + k[u]);
+        for (int s = 0; s < YA_STAGES - 1; ++s) issue(s);
+        for (int s = 0; s * YA_TERMS < nc; ++s) {
+            cp_async_wait<YA_STAGES - 2>();
+            __syncwarp(); // the warp's y_k are in, and its stage s - 1 is read
+            issue(s + YA_STAGES - 1);
+            const int slot = s % YA_STAGES * YA_TERMS;
+            auto term = [&](int u) {
+                const double2 a = ring[(slot + u) * YA_THREADS], b = yr[slot + u];
+                return dd_mul(dd_make(a.x, a.y), dd_make(b.x, b.y));
+            };
+            if ((s + 1) * YA_TERMS <= nc) {
+#pragma unroll
+                for (int u = 0; u < YA_TERMS; ++u) acc = dd_acc(acc, term(u));
+            } else {
+                for (int u = 0; s * YA_TERMS + u < nc; ++u) acc = dd_acc(acc, term(u));
             }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) acc = dd_acc(acc, dd_mul(a[u], b[u]));
         }
-        for (; t < v.nc; ++t) acc = dd_acc(acc, dd_mul(ld_dd(v.dense + v.dense_off[t] + e), ld_dd(y + v.con[t])));
+        cp_async_wait<0>();
+        if (e >= ne) return;
     } else {
+        if (e >= ne) return;
         for (int q = v.el_ptr[e]; q < v.el_ptr[e + 1]; ++q) acc = dd_acc(acc, dd_mul(v.el_val[q], ld_dd(y + v.el_con[q])));
     }
     dd_t r = dd_mul(MONE, acc);
     if (mode == 0) {
-        if (D) r = dd_acc(r, dd_mul(ONE, ld_dd(D + e)));
+        if (D) r = dd_acc(r, dd_mul(ONE, ld_dd(D + base + e)));
     } else {
         if (v.c_present) {
             if (v.c_dense) {
@@ -218,21 +248,26 @@ __global__ void sum_yA_kernel(const BlockView *views, int first, long nn, const 
                 for (int q = v.c_el_ptr[e]; q < v.c_el_ptr[e + 1]; ++q) r = dd_acc(r, dd_mul(v.c_el_val[q], ONE));
             }
         }
-        r = dd_acc(r, dd_mul(MONE, ld_dd(Z + e)));
+        r = dd_acc(r, dd_mul(MONE, ld_dd(Z + base + e)));
     }
-    st_dd(out + e, r);
+    st_dd(out + base + e, r);
 }
 
 void sum_yA(Context &c, const dd_t *y, Space &out, int mode, const Space *D, const Space *Z) {
-    for (const BlockRun &r : c.runs) {
-        const long nn = (long)r.n * r.n;
-        for (int b0 = 0; b0 < r.count; b0 += MAX_GRID_YZ) {
-            const int l = r.first + b0;
-            sum_yA_kernel<<<dim3(ceil_div(nn, 128), std::min(MAX_GRID_YZ, r.count - b0)), 128, 0, c.stream>>>(
-                c.views.p, l, nn, y, out.blk(c.off, l), mode, D ? D->blk(c.off, l) : nullptr, Z ? Z->blk(c.off, l) : nullptr);
-            CK_LAUNCH();
-        }
+    // the ring only where some block uses it
+    size_t smem = 0;
+    for (auto &b : c.blocks)
+        if (b->all_dense && b->nc > 0) smem = YA_SMEM;
+    static thread_local bool attr[64] = {};
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    if (!attr[dev & 63]) {
+        CK(cudaFuncSetAttribute(sum_yA_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)YA_SMEM));
+        attr[dev & 63] = true;
     }
+    sum_yA_kernel<<<c.n_yA_tasks, YA_THREADS, smem, c.stream>>>(c.views.p, c.yA_tasks.p, c.d_off.p, y, out.buf.p, mode, D ? D->buf.p : nullptr,
+                                                               Z ? Z->buf.p : nullptr);
+    CK_LAUNCH();
 }
 
 // ------------------------------------------------------------ init point
