@@ -36,6 +36,7 @@
 #include <cstring>
 
 #include "blas.h"
+#include "tile16.cuh"
 #include "devops.cuh"
 #include "newton.h"
 
@@ -223,6 +224,32 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) core_pairs_kernel(const
     }
 }
 
+// The same in 16 x 16 tiles (tile16.cuh).
+__global__ void __launch_bounds__(T16_THREADS, T16_CTAS) core_pairs16_kernel(const CoreBatch *bt) {
+    __shared__ Tile16 S;
+    const long total = bt->tile_off[0][bt->count];
+    for (long u = blockIdx.x; u < total; u += gridDim.x) {
+        const int q = core_find(bt->tile_off[0], bt->count, u);
+        const CoreItem &it = bt->it[q];
+        const int m = it.m, ntc = (m + T16 - 1) / T16;
+        const long t = u - bt->tile_off[0][q];
+        const int r0 = (int)(t / ntc) * T16, d0 = (int)(t % ntc) * T16;
+        if (d0 > r0 + T16 - 1) continue; // above the diagonal (uniform in the CTA)
+        const long K = (long)it.n * it.n;
+        const dd_t *G = it.G, *A = it.A;
+        dd_t acc[2] = {dd_zero(), dd_zero()};
+        tile16_sum<true, true, false, false>(
+            S, K, [&](int i, long k) { return r0 + i < m ? *reinterpret_cast<const double2 *>(G + k + K * (r0 + i)) : make_double2(0.0, 0.0); },
+            [&](int j, long k) { return d0 + j < m ? *reinterpret_cast<const double2 *>(A + k + K * (d0 + j)) : make_double2(0.0, 0.0); }, acc);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int r = r0 + threadIdx.x / T16 + 8 * x, d = d0 + threadIdx.x % T16;
+            if (r >= m || d > r) continue;
+            core_badd(it.B, m, it.con[it.perm[r]], it.con[it.perm[d]], dd_acc(dd_zero(), acc[x]));
+        }
+    }
+}
+
 // In-place lower Cholesky of every problem's B, one CTA per problem,
 // right-looking column by column: pivot (sqrt, then the reciprocal
 // 1/L(j,j)), scaling of the column by it, then the update of the trailing
@@ -342,7 +369,7 @@ CoreEngine::CoreEngine(int device) : p(new Impl) {
     core_fg_kernel<<<4 * p->sms, 256, 0, p->stream>>>(p->db, 0);
     core_fg_kernel<<<4 * p->sms, 256, 0, p->stream>>>(p->db, 1);
     cudaEventRecordWithFlags(p->ev_shape[0][0], p->stream, cudaEventRecordExternal);
-    core_pairs_kernel<0, 16, 16, 32, 1, 1><<<8 * p->sms, 256, 0, p->stream>>>(p->db);
+    core_pairs16_kernel<<<8 * p->sms, T16_THREADS, 0, p->stream>>>(p->db);
     cudaEventRecordWithFlags(p->ev_shape[0][1], p->stream, cudaEventRecordExternal);
     cudaEventRecordWithFlags(p->ev_shape[1][0], p->stream, cudaEventRecordExternal);
     core_pairs_kernel<1, 32, 32, 16, 2, 2><<<4 * p->sms, 256, 0, p->stream>>>(p->db);

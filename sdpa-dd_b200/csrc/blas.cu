@@ -22,6 +22,7 @@
 #include "devops.cuh"
 #include "ozaki.h"
 #include "prof.h"
+#include "tile16.cuh"
 
 #include <algorithm>
 
@@ -35,20 +36,31 @@ namespace sddd {
 // by alpha as it is staged ("temp = alpha * B(l,j)"), then c += temp * a
 // from the (beta-scaled) C; GEMM_AB_POST (Rgemm_TN/TT_omp): the products
 // are summed from zero and C += alpha * sum.
-template <int BM, int BN, int BK, int TM, int TN, bool TA, bool TB, int MODE>
+// STACK: the rows of A and C are those of M / stack matrices of `stack` rows,
+// one after the other, matrix r at A + r sA and C + r sC.
+template <int BM, int BN, int BK, int TM, int TN, bool TA, bool TB, int MODE, bool STACK = false>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
     gemm_kernel(int M, int N, int K, const dd_t *__restrict__ A, long lda, long sA, const dd_t *__restrict__ B, long ldb, long sB, dd_t *C,
-                long ldc, long sC, int lower, dd_t alpha) {
+                long ldc, long sC, int lower, dd_t alpha, int stack) {
+    static_assert(!STACK || (!TA && MODE == GEMM_STORE), "the stacked form is A_r B");
     constexpr int TX = BN / TN, TY = BM / TM, NT = TX * TY;
     __shared__ double2 As[BK][BM + 1];
     __shared__ double2 Bs[BK][BN + 1];
+    __shared__ long arow[STACK ? BM : 1]; // a row's offset in A
     const long bz = blockIdx.z;
-    A += bz * sA;
+    if (!STACK) {
+        A += bz * sA;
+        C += bz * sC;
+    }
     B += bz * sB;
-    C += bz * sC;
-    const int i0 = blockIdx.y * BM, j0 = blockIdx.x * BN;
+    // (the long dimension of a stacked product is on grid.x)
+    const int i0 = (STACK ? blockIdx.x : blockIdx.y) * BM, j0 = (STACK ? blockIdx.y : blockIdx.x) * BN;
     if (lower && i0 + BM <= j0) return; // tile entirely above the diagonal
     const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+    if (STACK) {
+        for (int e = tid; e < BM; e += NT) arow[e] = (i0 + e) / stack * sA + (i0 + e) % stack;
+        __syncthreads();
+    }
     dd_t acc[TM][TN];
 #pragma unroll
     for (int r = 0; r < TM; ++r)
@@ -72,7 +84,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
             }
             int gi = i0 + ii, gk = k0 + kk;
             double2 v = make_double2(0.0, 0.0);
-            if (gi < M && gk < K) v = *reinterpret_cast<const double2 *>(TA ? A + gk + lda * (long)gi : A + gi + lda * (long)gk);
+            if (gi < M && gk < K) v = *reinterpret_cast<const double2 *>(TA ? A + gk + lda * (long)gi : A + (STACK ? arow[ii] : gi) + lda * (long)gk);
             As[kk][ii] = v;
         }
         for (int e = tid; e < BN * BK; e += NT) {
@@ -123,33 +135,119 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
         for (int c = 0; c < TN; ++c) {
             int gi = i0 + ty + TY * r, gj = j0 + tx + TX * c;
             if (gi < M && gj < N && (!lower || gi >= gj)) {
-                dd_t *cp = C + gi + ldc * (long)gj;
+                dd_t *cp = C + (STACK ? gi / stack * sC + gi % stack : gi) + ldc * (long)gj;
                 st_dd(cp, MODE == GEMM_AB_POST ? dd_acc(ld_dd(cp), dd_mul(alpha, acc[r][c])) : acc[r][c]);
             }
         }
 }
 
-// 64 x 64 tiles (4 x 4 entries a thread) when they fill the GPU; for
-// small products (fewer 64 x 64 tiles than half the SMs) 16 x 16 tiles
-// with one entry a thread, so the work spreads over more SMs.  Each
-// entry's k-order is the same either way.
+// The same in 16 x 16 tiles (tile16.cuh).  Order 500: 183 us, the FP64 work
+// alone 134; one entry a thread, 256 threads, took 204.
+template <bool TA, bool TB, int MODE, bool PIPE>
+__global__ void __launch_bounds__(T16_THREADS, T16_CTAS)
+    gemm16_kernel(int M, int N, int K, const dd_t *__restrict__ A, long lda, long sA, const dd_t *__restrict__ B, long ldb, long sB, dd_t *C, long ldc,
+                  long sC, int lower, dd_t alpha) {
+    __shared__ Tile16 S;
+    const long bz = blockIdx.z;
+    A += bz * sA;
+    B += bz * sB;
+    C += bz * sC;
+    const int i0 = blockIdx.y * T16, j0 = blockIdx.x * T16;
+    if (lower && i0 + T16 <= j0) return; // tile entirely above the diagonal
+    const int gj = j0 + threadIdx.x % T16, gi = i0 + threadIdx.x / T16;
+    dd_t acc[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+        acc[r] = (MODE == GEMM_STORE || MODE == GEMM_AB_POST || gi + 8 * r >= M || gj >= N) ? dd_zero() : ld_dd(C + gi + 8 * r + ldc * (long)gj);
+    tile16_sum<TA, !TB, MODE == GEMM_SUB, PIPE>(
+        S, K,
+        [&](int i, long k) {
+            return i0 + i < M ? *reinterpret_cast<const double2 *>(TA ? A + k + lda * (long)(i0 + i) : A + i0 + i + lda * k) : make_double2(0.0, 0.0);
+        },
+        [&](int j, long k) {
+            if (j0 + j >= N) return make_double2(0.0, 0.0);
+            const double2 v = *reinterpret_cast<const double2 *>(TB ? B + j0 + j + ldb * k : B + k + ldb * (long)(j0 + j));
+            if (MODE != GEMM_AB_PRE) return v;
+            const dd_t t = dd_mul(alpha, dd_make(v.x, v.y));
+            return make_double2(t.hi, t.lo);
+        },
+        acc);
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+        if (gi + 8 * r < M && gj < N && (!lower || gi + 8 * r >= gj)) {
+            dd_t *cp = C + gi + 8 * r + ldc * (long)gj;
+            st_dd(cp, MODE == GEMM_AB_POST ? dd_acc(ld_dd(cp), dd_mul(alpha, acc[r])) : acc[r]);
+        }
+}
+
+// 64 x 64 tiles (4 x 4 entries a thread) when they fill the GPU; 16 x 16
+// tiles for small products (fewer 64 x 64 tiles than half the SMs), so that
+// the work spreads over more SMs, and where the larger tiles would be mostly
+// padding (16 x 16 tiles run at about 0.7 of the FP64 rate, 64 x 64 at 0.9;
+// 200 products of order 20: 33 us in 64 x 64 tiles,
+// 9 in 16 x 16).  Each entry's k-order is the same either way.
 constexpr long GEMM_SMALL_TILES = 74;
 template <bool TA, bool TB, int MODE>
 static void gemm_launch(cudaStream_t st, int M, int N, int K, const dd_t *A, long lda, long sA, const dd_t *B, long ldb, long sB, dd_t *C, long ldc,
                         long sC, int batch, bool lower, dd_t alpha = dd_t{1.0, 0.0}) {
-    if ((long)ceil_div(N, 64) * ceil_div(M, 64) * batch < GEMM_SMALL_TILES) {
-        constexpr int BM = 16, BN = 16, BK = 16, TM = 1, TN = 1;
-        dim3 grid(ceil_div(N, BN), ceil_div(M, BM), batch);
-        gemm_kernel<BM, BN, BK, TM, TN, TA, TB, MODE>
-            <<<grid, (BM / TM) * (BN / TN), 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, lower ? 1 : 0, alpha);
+    const long m16 = ceil_div(M, T16), n16 = ceil_div(N, T16), m64 = ceil_div(M, 64), n64 = ceil_div(N, 64);
+    if (m64 * n64 * batch < GEMM_SMALL_TILES || 13 * m16 * n16 < 10 * 16 * m64 * n64) {
+        dim3 grid((unsigned)n16, (unsigned)m16, batch);
+        if (m16 * n16 * batch <= T16_PIPE_TILES)
+            gemm16_kernel<TA, TB, MODE, true><<<grid, T16_THREADS, 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, lower ? 1 : 0, alpha);
+        else
+            gemm16_kernel<TA, TB, MODE, false><<<grid, T16_THREADS, 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, lower ? 1 : 0, alpha);
         CK_LAUNCH();
         return;
     }
     constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
-    dim3 grid(ceil_div(N, BN), ceil_div(M, BM), batch);
+    dim3 grid((unsigned)n64, (unsigned)m64, batch);
     gemm_kernel<BM, BN, BK, TM, TN, TA, TB, MODE>
-        <<<grid, (BM / TM) * (BN / TN), 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, lower ? 1 : 0, alpha);
+        <<<grid, (BM / TM) * (BN / TN), 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, lower ? 1 : 0, alpha, 0);
     CK_LAUNCH();
+}
+
+// C_r = A_r B (rows) or C_r = A B_r of `count` matrices of order n that lie
+// n^2 apart, as one product whose long dimension runs through the matrices,
+// so that only the other one is padded; its tile is 4 TS wide, TS threads of
+// four entries, TS as the order wants it.
+template <int TS> static void stacked_launch(cudaStream_t st, bool rows, int n, int count, const dd_t *A, const dd_t *B, dd_t *C) {
+    constexpr int BS = 4 * TS, BL = 64, BK = 16;
+    const long nn = (long)n * n;
+    const dd_t one = {1.0, 0.0};
+    const unsigned tl = ceil_div((long)n * count, BL), ts = ceil_div(n, BS);
+    if (rows)
+        gemm_kernel<BL, BS, BK, 4, 4, false, false, GEMM_STORE, true>
+            <<<dim3(tl, ts), 16 * TS, 0, st>>>(n * count, n, n, A, n, nn, B, n, 0, C, n, nn, 0, one, n);
+    else
+        gemm_kernel<BS, BL, BK, 4, 4, false, false, GEMM_STORE>
+            <<<dim3(tl, ts), 16 * TS, 0, st>>>(n, n * count, n, A, n, 0, B, n, 0, C, n, 0, 0, one, 0);
+    CK_LAUNCH();
+}
+void gemm_stacked(cudaStream_t st, bool rows, int n, int count, const dd_t *A, const dd_t *B, dd_t *C) {
+    if (n <= 0 || count <= 0) return;
+    // the fewest warps over the short dimension, then the fewest tiles
+    int ts = 8, best = 1 << 30;
+    for (int t = 16; t >= 8; --t) {
+        const int tiles = (int)ceil_div(n, 4 * t), cost = tiles * (int)ceil_div(16 * t, 32);
+        if (cost < best) best = cost, ts = t;
+    }
+    const long nn = (long)n * n;
+    if ((long)n * count > (1L << 30) || (long)ceil_div((long)n * count, 64) * ceil_div(n, 4 * ts) < 2 * GEMM_SMALL_TILES) {
+        gemm(st, 'N', 'N', GEMM_STORE, n, n, n, A, n, rows ? nn : 0, B, n, rows ? 0 : nn, C, n, nn, count, false);
+        return;
+    }
+    switch (ts) {
+    case 8: stacked_launch<8>(st, rows, n, count, A, B, C); break;
+    case 9: stacked_launch<9>(st, rows, n, count, A, B, C); break;
+    case 10: stacked_launch<10>(st, rows, n, count, A, B, C); break;
+    case 11: stacked_launch<11>(st, rows, n, count, A, B, C); break;
+    case 12: stacked_launch<12>(st, rows, n, count, A, B, C); break;
+    case 13: stacked_launch<13>(st, rows, n, count, A, B, C); break;
+    case 14: stacked_launch<14>(st, rows, n, count, A, B, C); break;
+    case 15: stacked_launch<15>(st, rows, n, count, A, B, C); break;
+    default: stacked_launch<16>(st, rows, n, count, A, B, C);
+    }
 }
 
 // C = beta C as Rgemm's first loop: zero for beta == 0, unchanged for

@@ -16,6 +16,9 @@ constexpr int MAX_GRID_YZ = 65535; // largest grid.y / grid.z of one launch
 // only.  op: 'N' or 'T'.
 void gemm(cudaStream_t st, char ta, char tb, int mode, int M, int N, int K, const dd_t *A, long lda, long sA, const dd_t *B, long ldb, long sB,
           dd_t *C, long ldc, long sC, int batch, bool lower);
+// C_r = A_r B (rows) or C_r = A B_r for r < count, order n, the matrices of
+// the stacked operand and of C n^2 apart: gemm's STORE form, entry by entry.
+void gemm_stacked(cudaStream_t st, bool rows, int n, int count, const dd_t *A, const dd_t *B, dd_t *C);
 // In-place lower Cholesky; *info_dev = 0 or the failing 1-based column.
 // rdiag_dev holds POTRF_NB dd of scratch.  With tc, the trailing updates
 // run as tensor-core slice products (ozaki.h) instead of dd GEMMs.

@@ -378,6 +378,18 @@ static void build_block(Context &c, const Problem &P, int l, BlockDev &bd) {
     bd.ownFG.upload(bd.h_ownFG, st);
     bd.ownF3.upload(bd.h_ownF3, st);
     bd.fg_index.upload(fg_index, st);
+    {
+        std::vector<int2> tiles;
+        const int nfg = bd.nFG(), nt = (int)ceil_div(ndense, 16);
+        if (pairs_small(nfg, ndense))
+            for (int r0 = 0; r0 < nfg; r0 += 16) {
+                // partners of sorted position up to the tile's last owner
+                const int lim = bd.h_ownFG[std::min(r0 + 16, nfg) - 1] - bd.nsparse;
+                for (int t = 0; t < nt && 16 * t <= lim; ++t) tiles.push_back(make_int2(r0 / 16, t));
+            }
+        bd.n_pair_tiles = (int)tiles.size();
+        bd.pair_tiles.upload(tiles, st);
+    }
     bd.fg_dense_contig = !bd.h_ownFG.empty();
     for (size_t r = 0; r < bd.h_ownFG.size(); ++r) {
         int t = perm[bd.h_ownFG[r]];

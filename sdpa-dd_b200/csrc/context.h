@@ -110,6 +110,8 @@ struct BlockDev {
     DBuf<int> ownFG, ownF3;
     DBuf<int> fg_index;  // [s] -> index in ownFG or -1
     bool fg_dense_contig = false; // all FG owners dense and contiguous in t
+    DBuf<int2> pair_tiles; // 16 x 16 tiles of (owner, dense partner) that hold a pair, when they go by such tiles
+    int n_pair_tiles = 0;
     // F = A_i Z^-1 for sparse FG owners as row lists: row i of F is the
     // ordered sum of v * (row src of Z^-1) (Raxpy row updates,
     // sdpa_linear.cpp:832-893); per owner r: rl_off[r] into rl_ptr (n+1)
@@ -158,6 +160,9 @@ struct SchurGraph {
 struct BlockRun {
     int first, count, n;
 };
+
+// Few pairs of FG owners and dense partners (schur.cu): 16 x 16 tiles.
+inline bool pairs_small(int nfg, int ndense) { return (long)ceil_div(ndense, 64) * ceil_div(nfg, 64) < 2L * 148; }
 
 struct Context {
     int device = 0;

@@ -24,6 +24,7 @@
 #include "newton.h"
 #include "devops.cuh"
 #include "prof.h"
+#include "tile16.cuh"
 
 #include <algorithm>
 #include <unordered_map>
@@ -143,6 +144,32 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
             // acc holds the Rdot partial (templ); Rdot returns 0 + templ
             pair_out(B, m, stage, bv.nc, s_own, s_par, i, j, dd_acc(dd_zero(), acc[r][c]));
         }
+}
+
+// The same in 16 x 16 tiles (tile16.cuh), one CTA for each tile that holds a
+// valid pair (tiles[]: row tile, partner tile).  Only those are launched:
+// where a square grid's empty CTAs ended at once, the others shared SMs
+// (m = 200: 667 us, some SMs with three tiles; 91 CTAs alone 430).
+template <bool PIPE>
+__global__ void __launch_bounds__(T16_THREADS, T16_CTAS) schur_dense_pairs16_kernel(BlockView bv, const int2 *tiles, const int *ownFG, int nfg,
+                                                                                   int ndense, const dd_t *__restrict__ W,
+                                                                                   const dd_t *__restrict__ V, dd_t *B, int m, dd_t *stage) {
+    __shared__ Tile16 S;
+    const long K = (long)bv.n * bv.n;
+    const int r0 = tiles[blockIdx.x].x * T16, d0 = tiles[blockIdx.x].y * T16;
+    const int gd = d0 + threadIdx.x % T16, gr = r0 + threadIdx.x / T16;
+    dd_t acc[2] = {dd_zero(), dd_zero()};
+    tile16_sum<true, true, false, PIPE>(
+        S, K, [&](int i, long k) { return r0 + i < nfg ? *reinterpret_cast<const double2 *>(W + k + K * (r0 + i)) : make_double2(0.0, 0.0); },
+        [&](int j, long k) { return d0 + j < ndense ? *reinterpret_cast<const double2 *>(V + k + K * (d0 + j)) : make_double2(0.0, 0.0); }, acc);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        if (gr + 8 * r >= nfg || gd >= ndense) continue;
+        const int s_own = ownFG[gr + 8 * r], s_par = bv.nsparse + gd;
+        if (s_par > s_own) continue;
+        // acc holds the Rdot partial (templ); Rdot returns 0 + templ
+        pair_out(B, m, stage, bv.nc, s_own, s_par, bv.con[bv.perm[s_own]], bv.con[bv.perm[s_par]], dd_acc(dd_zero(), acc[r]));
+    }
 }
 
 // ------------------------------------------ sparse partners of F1 owners
@@ -280,7 +307,7 @@ static void schur_block(Context &c, int l, cudaStream_t st, dd_t *Fb, dd_t *Gb, 
         if (bd.fg_dense_contig) {
             // the FG owners' dense matrices are consecutive in bd.dense
             const long o0 = bd.h_dense_off[bd.h_perm[bd.h_ownFG[0]]];
-            gemm(st, 'N', 'N', GEMM_STORE, n, n, n, bd.dense.p + o0, n, nn, Zi, n, 0, Fb, n, nn, nfg, false);
+            gemm_stacked(st, true, n, nfg, bd.dense.p + o0, Zi, Fb);
         } else {
             for (int r = 0; r < nfg; ++r) {
                 long o = bd.h_dense_off[bd.h_perm[bd.h_ownFG[r]]];
@@ -288,7 +315,7 @@ static void schur_block(Context &c, int l, cudaStream_t st, dd_t *Fb, dd_t *Gb, 
             }
         }
         // G_r = X F_r
-        gemm(st, 'N', 'N', GEMM_STORE, n, n, n, X, n, 0, Fb, n, nn, Gb, n, nn, nfg, false);
+        gemm_stacked(st, false, n, nfg, X, Fb, Gb);
         // dense partners
         const int ndense = bd.nc - bd.nsparse;
         if (!stage && c.tc_slices > 0 && bd.nsparse == 0 && nfg == bd.nc && bd.fg_dense_contig && nn <= OG_MAX_K) {
@@ -305,18 +332,18 @@ static void schur_block(Context &c, int l, cudaStream_t st, dd_t *Fb, dd_t *Gb, 
         } else if (ndense > 0) {
             // Every pair is one sequential dot over the n^2 entries.  With
             // few pairs (small m) 64 x 64 tiles of 16 pairs per thread
-            // leave the GPU nearly idle on long chains; one pair per
-            // thread in 16 x 16 tiles spreads them over many more CTAs.
-            if ((long)ceil_div(ndense, 64) * ceil_div(nfg, 64) >= 2L * 148) {
+            // leave the GPU nearly idle on long chains; two pairs per
+            // thread in 16 x 16 tiles spread them over many more CTAs.
+            if (!pairs_small(nfg, ndense)) {
                 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
                 dim3 grid(ceil_div(ndense, BN), ceil_div(nfg, BM));
                 schur_dense_pairs_kernel<BM, BN, BK, TM, TN>
                     <<<grid, (BM / TM) * (BN / TN), 0, st>>>(bv, bd.ownFG.p, nfg, ndense, Gb, bd.dense.p, c.B.p, m, stage);
             } else {
-                constexpr int BM = 16, BN = 16, BK = 32, TM = 1, TN = 1;
-                dim3 grid(ceil_div(ndense, BN), ceil_div(nfg, BM));
-                schur_dense_pairs_kernel<BM, BN, BK, TM, TN>
-                    <<<grid, (BM / TM) * (BN / TN), 0, st>>>(bv, bd.ownFG.p, nfg, ndense, Gb, bd.dense.p, c.B.p, m, stage);
+                // (stage: the blocks' launches share the GPU)
+                auto *kernel = !stage && bd.n_pair_tiles <= T16_PIPE_TILES ? schur_dense_pairs16_kernel<true> : schur_dense_pairs16_kernel<false>;
+                if (bd.n_pair_tiles > 0)
+                    kernel<<<bd.n_pair_tiles, T16_THREADS, 0, st>>>(bv, bd.pair_tiles.p, bd.ownFG.p, nfg, ndense, Gb, bd.dense.p, c.B.p, m, stage);
             }
             CK_LAUNCH();
         }
