@@ -54,7 +54,10 @@ struct TrsvSync {
 // x = L^-1 x ('N') or L^-T x ('T'), L lower, as Rtrsv("Lower", trans, "NonUnit").
 // shared_gpu: other streams keep the GPU busy (a batch worker); short
 // solves then run in one CTA with an ordinary launch.
-void trsv_lower(cudaStream_t st, char trans, const dd_t *L, long lda, int n, dd_t *x, TrsvSync &sync, bool shared_gpu = false);
+// nrhs right-hand sides, ldx apart, side by side (the sync object holds flags
+// for all of them).
+void trsv_lower(cudaStream_t st, char trans, const dd_t *L, long lda, int n, dd_t *x, TrsvSync &sync, bool shared_gpu = false, int nrhs = 1,
+                long ldx = 0);
 // Throws when a solve since the flags were zeroed gave up waiting
 // (synchronises st).
 void trsv_check(cudaStream_t st, const TrsvSync &sync);

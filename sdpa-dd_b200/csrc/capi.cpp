@@ -774,7 +774,9 @@ int sddd_Rpotrs(sddd_ctx *ctx, char uplo, long n, long nrhs, const sddd_dd *A, l
         if (n == 0 || nrhs == 0) return SDDD_OK;
         sddd::Context &c = *ctx->c;
         const dd_t *L = reinterpret_cast<const dd_t *>(A);
-        sddd::TrsvSync &sync = sddd::trsv_sync(c, (int)n);
+        // plain form: groups of right-hand sides side by side, a few CTAs each
+        const int group = c.tc_slices > 0 ? 1 : (int)std::min(nrhs, 8L);
+        sddd::TrsvSync &sync = sddd::trsv_sync(c, (int)n, group);
         if (c.tc_slices > 0) {
             // the split form's blocked solves; the inverted diagonal blocks
             // take the context's buffer (a Newton solve in progress
@@ -788,10 +790,11 @@ int sddd_Rpotrs(sddd_ctx *ctx, char uplo, long n, long nrhs, const sddd_dd *A, l
                 sddd::trsv_blocked(c.stream, 'T', L, lda, (int)n, c.trsv_winv.p, x, sync);
             }
         } else {
-            for (long r = 0; r < nrhs; ++r) {
+            for (long r = 0; r < nrhs; r += group) {
                 dd_t *x = reinterpret_cast<dd_t *>(B) + ldb * r;
-                sddd::trsv_lower(c.stream, 'N', L, lda, (int)n, x, sync);
-                sddd::trsv_lower(c.stream, 'T', L, lda, (int)n, x, sync);
+                const int g = (int)std::min<long>(group, nrhs - r);
+                sddd::trsv_lower(c.stream, 'N', L, lda, (int)n, x, sync, false, g, ldb);
+                sddd::trsv_lower(c.stream, 'T', L, lda, (int)n, x, sync, false, g, ldb);
             }
         }
         sddd::trsv_check(c.stream, sync);

@@ -151,8 +151,8 @@ OzakiGemmWork &tcg_work(Context &c, int n, long K, int slices) {
     return c.tcg;
 }
 
-TrsvSync &trsv_sync(Context &c, int n) {
-    const int nblk = (int)ceil_div(n, 64);
+TrsvSync &trsv_sync(Context &c, int n, int nrhs) {
+    const int nblk = (int)ceil_div(n, 64) * nrhs;
     if (nblk > c.trsv.capacity || !c.trsv.flags) {
         CK(cudaStreamSynchronize(c.stream));
         c.trsv_flags.alloc((size_t)nblk + 1);

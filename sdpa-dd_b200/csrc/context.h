@@ -300,8 +300,9 @@ struct Context {
 Context *create_context(int device);
 void upload_problem(Context &c, Problem &&p);
 void alloc_state(Context &c);
-// The triangular-solve progress words, grown (and zeroed) to cover order n.
-TrsvSync &trsv_sync(Context &c, int n);
+// The triangular-solve progress words, grown (and zeroed) to cover nrhs
+// right-hand sides of order n.
+TrsvSync &trsv_sync(Context &c, int n, int nrhs = 1);
 // The split workspace for an order-n factorisation with `slices` slices
 // (grown as needed).
 OzakiWork &tc_work(Context &c, int n, int slices);
