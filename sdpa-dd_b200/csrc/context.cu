@@ -379,7 +379,8 @@ static void build_block(Context &c, const Problem &P, int l, BlockDev &bd) {
     bd.ownF3.upload(bd.h_ownF3, st);
     bd.fg_index.upload(fg_index, st);
     {
-        std::vector<int2> tiles;
+        std::vector<int2> &tiles = bd.h_pair_tiles;
+        tiles.clear();
         const int nfg = bd.nFG(), nt = (int)ceil_div(ndense, 16);
         if (pairs_small(nfg, ndense))
             for (int r0 = 0; r0 < nfg; r0 += 16) {
@@ -388,7 +389,6 @@ static void build_block(Context &c, const Problem &P, int l, BlockDev &bd) {
                 for (int t = 0; t < nt && 16 * t <= lim; ++t) tiles.push_back(make_int2(r0 / 16, t));
             }
         bd.n_pair_tiles = (int)tiles.size();
-        bd.pair_tiles.upload(tiles, st);
     }
     bd.fg_dense_contig = !bd.h_ownFG.empty();
     for (size_t r = 0; r < bd.h_ownFG.size(); ++r) {
@@ -429,9 +429,20 @@ void upload_problem(Context &c, Problem &&p) {
     c.views.upload(views, c.stream);
     c.d_off.upload(c.off, c.stream);
     c.d_sizes.upload(c.sizes, c.stream);
+    // the tables, one after the other (pairs at even places)
+    std::vector<int> tab;
+    auto table_at = [&](const void *src, size_t ints) {
+        const size_t at = tab.size() + tab.size() % 2;
+        tab.resize(at + ints);
+        if (ints > 0) std::memcpy(tab.data() + at, src, ints * sizeof(int));
+        return at;
+    };
     std::vector<int> dim(c.nSDP + 1, 0);
     for (int l = 0; l < c.nSDP; ++l) dim[l + 1] = dim[l] + c.sizes[l];
-    c.d_dim.upload(dim, c.stream);
+    const size_t dim_at = table_at(dim.data(), dim.size());
+    std::vector<size_t> tiles_at;
+    for (auto &bd : c.blocks) tiles_at.push_back(table_at(bd->h_pair_tiles.data(), 2 * bd->h_pair_tiles.size()));
+    size_t task_at, t_at, pos_at, yA_at;
     std::vector<int> ptr(c.m + 1, 0), bl, tt;
     for (int k = 0; k < c.m; ++k) {
         for (auto &kv : P.A[k]) {
@@ -473,10 +484,10 @@ void upload_problem(Context &c, Problem &&p) {
         // long sums first
         std::stable_sort(tasks.begin(), tasks.end(), [&](const InnerTask &a, const InnerTask &b) { return c.sizes[a.block] > c.sizes[b.block]; });
         c.n_inner_tasks = (int)tasks.size();
-        c.inner_tasks.upload(tasks, c.stream);
-        c.inner_t.upload(it, c.stream);
-        c.inner_at.upload(at, c.stream);
-        if (!tasks.empty()) c.inner_prod.alloc(bl.size());
+        static_assert(sizeof(InnerTask) == 3 * sizeof(int), "a table of ints");
+        task_at = table_at(tasks.data(), 3 * tasks.size());
+        t_at = table_at(it.data(), it.size());
+        pos_at = table_at(at.data(), at.size());
         for (int p : at) tt[p] = -1;
     }
     {
@@ -488,8 +499,16 @@ void upload_problem(Context &c, Problem &&p) {
         for (int l : order)
             for (long e = 0; e < (long)c.sizes[l] * c.sizes[l]; e += 128) tasks.push_back(make_int2(l, (int)(e / 128)));
         c.n_yA_tasks = (int)tasks.size();
-        c.yA_tasks.upload(tasks, c.stream);
+        yA_at = table_at(tasks.data(), 2 * tasks.size());
     }
+    c.tables.upload(tab, c.stream);
+    c.d_dim = c.tables.p + dim_at;
+    c.inner_tasks = reinterpret_cast<const InnerTask *>(c.tables.p + task_at);
+    c.inner_t = c.tables.p + t_at;
+    c.inner_at = c.tables.p + pos_at;
+    c.yA_tasks = reinterpret_cast<const int2 *>(c.tables.p + yA_at);
+    for (int l = 0; l < c.nSDP; ++l) c.blocks[l]->pair_tiles = reinterpret_cast<const int2 *>(c.tables.p + tiles_at[l]);
+    c.primalVec.alloc((size_t)c.m + (c.n_inner_tasks > 0 ? bl.size() : 0));
     c.cb_ptr.upload(ptr, c.stream);
     c.cb_block.upload(bl, c.stream);
     c.cb_t.upload(tt, c.stream);
@@ -509,7 +528,6 @@ void alloc_state(Context &c) {
     c.y.alloc(c.m);
     c.Dy.alloc(c.m);
     c.g.alloc(c.m);
-    c.primalVec.alloc(c.m);
     c.B.alloc((size_t)c.m * c.m);
     size_t fg = 0;
     for (auto &bd : c.blocks) fg = std::max(fg, (size_t)bd->nFG() * bd->n * bd->n);

@@ -110,7 +110,10 @@ struct BlockDev {
     DBuf<int> ownFG, ownF3;
     DBuf<int> fg_index;  // [s] -> index in ownFG or -1
     bool fg_dense_contig = false; // all FG owners dense and contiguous in t
-    DBuf<int2> pair_tiles; // 16 x 16 tiles of (owner, dense partner) that hold a pair, when they go by such tiles
+    // 16 x 16 tiles of (owner, dense partner) that hold a pair, when they go
+    // by such tiles (in the context's tables)
+    std::vector<int2> h_pair_tiles;
+    const int2 *pair_tiles = nullptr;
     int n_pair_tiles = 0;
     // F = A_i Z^-1 for sparse FG owners as row lists: row i of F is the
     // ordered sum of v * (row src of Z^-1) (Raxpy row updates,
@@ -202,19 +205,22 @@ struct Context {
     DBuf<BlockView> views; // [l]
     DBuf<long> d_off;      // [l] block offsets within a space
     DBuf<int> d_sizes;     // [l] block sizes
-    DBuf<int> d_dim;       // [l] rows before block l; [nSDP] all rows
     // per constraint: (block, t) pairs ascending by block
     // (t = -1: the product is formed by a task, below)
     DBuf<int> cb_ptr, cb_block, cb_t;
     // the tasks of constraint_inner, their matrices (t in the block, position
     // in cb_*), grouped by block, and the products by position
-    DBuf<InnerTask> inner_tasks;
-    DBuf<int> inner_t, inner_at;
-    DBuf<dd_t> inner_prod;
+    // (the tables below lie in one buffer, the products behind primalVec:
+    // an allocation costs about 0.1 ms)
+    const InnerTask *inner_tasks = nullptr;
+    const int *inner_t = nullptr, *inner_at = nullptr;
+    dd_t *inner_prod() const { return primalVec.p + m; }
     int n_inner_tasks = 0;
     // (block, 128-entry chunk) of each CTA of sum_k y_k A_k
-    DBuf<int2> yA_tasks;
+    const int2 *yA_tasks = nullptr;
     int n_yA_tasks = 0;
+    const int *d_dim = nullptr; // [l] rows before block l; [nSDP] all rows
+    DBuf<int> tables;
     DBuf<dd_t> b;
     // iterate and derived (Solutions)
     Space X, Z, invCholX, invCholZ, invZ;
@@ -225,7 +231,7 @@ struct Context {
     DBuf<dd_t> B;   // m x m Schur matrix, factored in place
     // Residuals
     Space dualMat;
-    DBuf<dd_t> primalVec;
+    DBuf<dd_t> primalVec; // m entries, then constraint_inner's products
     // WorkVariables
     Space W1, W2;
     // Schur work: F_i and G_i of FG owners (largest block)

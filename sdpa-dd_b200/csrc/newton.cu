@@ -159,12 +159,12 @@ void constraint_inner(Context &c, const Space &M, const dd_t *addv, dd_t *out) {
             CK(cudaFuncSetAttribute(inner_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IP_SMEM));
             attr[dev & 63] = true;
         }
-        inner_pairs_kernel<<<c.n_inner_tasks, IP_THREADS, IP_SMEM, c.stream>>>(c.inner_tasks.p, c.inner_t.p, c.inner_at.p, c.views.p, c.d_off.p, M.buf.p,
-                                                                      c.inner_prod.p);
+        inner_pairs_kernel<<<c.n_inner_tasks, IP_THREADS, IP_SMEM, c.stream>>>(c.inner_tasks, c.inner_t, c.inner_at, c.views.p, c.d_off.p, M.buf.p,
+                                                                      c.inner_prod());
         CK_LAUNCH();
     }
     constraint_inner_kernel<<<ceil_div(c.m, 64), 64, 0, c.stream>>>(c.m, c.views.p, c.d_off.p, c.cb_ptr.p, c.cb_block.p, c.cb_t.p, M.buf.p,
-                                                                    c.inner_prod.p, addv, out);
+                                                                    c.inner_prod(), addv, out);
     CK_LAUNCH();
 }
 
@@ -265,7 +265,7 @@ void sum_yA(Context &c, const dd_t *y, Space &out, int mode, const Space *D, con
         CK(cudaFuncSetAttribute(sum_yA_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)YA_SMEM));
         attr[dev & 63] = true;
     }
-    sum_yA_kernel<<<c.n_yA_tasks, YA_THREADS, smem, c.stream>>>(c.views.p, c.yA_tasks.p, c.d_off.p, y, out.buf.p, mode, D ? D->buf.p : nullptr,
+    sum_yA_kernel<<<c.n_yA_tasks, YA_THREADS, smem, c.stream>>>(c.views.p, c.yA_tasks, c.d_off.p, y, out.buf.p, mode, D ? D->buf.p : nullptr,
                                                                Z ? Z->buf.p : nullptr);
     CK_LAUNCH();
 }
@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS) lambda_trace_kernel(const dd_t 
 
 int ScalarBatch::lambda_trace(const Space &s, double lambda) {
     const int g = group(1);
-    lambda_trace_kernel<<<1, CHAIN_THREADS, 0, c.stream>>>(s.buf.p, c.d_off.p, c.d_dim.p, c.nSDP, lambda, c.scal.p + groups[g].first);
+    lambda_trace_kernel<<<1, CHAIN_THREADS, 0, c.stream>>>(s.buf.p, c.d_off.p, c.d_dim, c.nSDP, lambda, c.scal.p + groups[g].first);
     CK_LAUNCH();
     return g;
 }

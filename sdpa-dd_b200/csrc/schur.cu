@@ -343,7 +343,7 @@ static void schur_block(Context &c, int l, cudaStream_t st, dd_t *Fb, dd_t *Gb, 
                 // (stage: the blocks' launches share the GPU)
                 auto *kernel = !stage && bd.n_pair_tiles <= T16_PIPE_TILES ? schur_dense_pairs16_kernel<true> : schur_dense_pairs16_kernel<false>;
                 if (bd.n_pair_tiles > 0)
-                    kernel<<<bd.n_pair_tiles, T16_THREADS, 0, st>>>(bv, bd.pair_tiles.p, bd.ownFG.p, nfg, ndense, Gb, bd.dense.p, c.B.p, m, stage);
+                    kernel<<<bd.n_pair_tiles, T16_THREADS, 0, st>>>(bv, bd.pair_tiles, bd.ownFG.p, nfg, ndense, Gb, bd.dense.p, c.B.p, m, stage);
             }
             CK_LAUNCH();
         }
