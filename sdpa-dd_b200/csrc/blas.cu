@@ -320,19 +320,35 @@ void gemm(cudaStream_t st, char ta, char tb, int mode, int M, int N, int K, cons
 // On a non-positive or NaN pivot the 1-based global column goes to *info
 // and the block is left as it was (Rpotrf2's n = 1 test,
 // mplapack/Rpotrf2.cpp).  1/L(j,j) for the panel goes to rdiag.
-// Dataflow form, with no CTA-wide barrier between columns: warp w owns
-// columns w and w + 32 in registers (lane l holds rows j + l and j + l + 32
-// of column j).  When column k is final (pivot, scaling) its owner copies
-// it to shared memory and its 32 lanes arrive on column k's mbarrier;
-// every warp waits for that barrier, then subtracts column k's term from
-// its own columns right of k, the owner of column k + 1 taking that column
-// first and finishing it at once, so that one pivot follows the next
-// through a single warp.  Every entry sees the same operations in the same
-// order as the column-by-column form: x(i,j) -= L(j,k) L(i,k) for k
-// ascending, then the sqrt (diagonal) or the scaling by 1/L(j,j).
+//
+// The block's time is its chain of pivots (a dd square root and reciprocal, a
+// product and a subtraction a column), so warp 0 carries that chain, alone on
+// its SM sub-partition (warps 4, 8, .. have no work): with column k in
+// registers (lane i holds rows i and i + 32), its last term still to come, it
+// forms L(k,k) and 1/L(k,k) in all lanes and that term beside them, takes
+// column k + 1, forms the next pivot from L(k+1,k) = x(k+1,k) / L(k,k) in
+// every lane, and scales and publishes column k beside that.  The warps of the
+// other sub-partitions hold columns 2 .. nb-1 in registers, in pairs j + j' =
+// nb + 2 whose nb - 2 entries fill two slots a lane, subtract the published
+// columns' terms, and hand column j over once column j - 2's term is in.
+// Hand-overs are named barriers; every one is reached by all its warps, a bad
+// pivot included.  Every entry sees x(i,j) -= L(j,k) L(i,k) for k ascending,
+// then the sqrt or the scaling.
+// Measured for nb = 64: 48 us; with warps that took turns at the pivot, on
+// lane 0 and with the plain divisions, behind an mbarrier a column, 70 us.
+// The same behind mbarriers 57 us (a wake-up costs several hundred cycles),
+// behind polled flags 53 us (the polls take the issue slots of the warps at
+// work); a second warp for the columns 52 us (their hand-over waits for the
+// helpers' FP64 work either way); sub-blocks of 16 columns in warp 0's
+// registers 95 us.
 constexpr int DIAG_THREADS = 1024;
-constexpr unsigned long long POTRF_WAIT_NS = 2000000000ull; // one mbarrier wait, at most
-static_assert(POTRF_NB <= 64 && DIAG_THREADS == 1024, "two columns a warp, two rows a lane");
+constexpr int DIAG_HELPERS = 24;
+constexpr int DIAG_PAIRS = 2;   // pairs a helper holds at most
+constexpr unsigned long long POTRF_WAIT_NS = 2000000000ull; // one wait, at most
+static_assert(POTRF_NB <= 64 && DIAG_THREADS == 1024 && DIAG_HELPERS * DIAG_PAIRS >= POTRF_NB / 2, "two rows a lane; warps 1-3, 5-7, .. help");
+__device__ __forceinline__ dd_t shfl_dd(dd_t v, int src) {
+    return dd_make(__shfl_sync(0xffffffffu, v.hi, src), __shfl_sync(0xffffffffu, v.lo, src));
+}
 // Bounded wait for phase 0 of an mbarrier.
 __device__ __forceinline__ bool bar_wait0(uint64_t *b) {
     if (mbar_try_wait(b, 0)) return true;
@@ -343,112 +359,127 @@ __device__ __forceinline__ bool bar_wait0(uint64_t *b) {
 }
 __global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_kernel(dd_t *A, long lda, int nb, int c0, int *info, dd_t *rdiag, long sA) {
     extern __shared__ double2 sm[];
-    double2 *S = sm; // nb x nb, column-major: the final columns
-    __shared__ uint64_t bar[POTRF_NB];
-    __shared__ int fail;
+    double2 *S = sm; // nb x nb, column-major: columns on their way, then final
+    __shared__ int stop; // k + 1: bad pivot k
     A += blockIdx.x * sA; // CTA b: matrix b of a batch of equal blocks (rdiag null then)
     if (*info != 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid < nb) mbar_init(&bar[tid], 32);
-    if (tid == 0) fail = 0;
-    __syncthreads();
-    volatile int *vfail = &fail;
-    dd_t x[2][2];
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int j = warp + 32 * c, i = j + lane + 32 * r;
-            x[c][r] = (j < nb && i < nb) ? ld_dd(A + (c0 + i) + lda * (long)(c0 + j)) : dd_from(0.0);
-        }
-    // Column warp + 32 c: pivot (lane 0 holds the diagonal), scaling, copy
-    // to shared memory, arrival.  False when the pivot fails.
-    auto finish = [&](const int c) -> bool {
-        const int j = warp + 32 * c;
-        int bad = 0;
-        double rh = 0.0, rl = 0.0;
-        if (lane == 0) {
-            const dd_t d = x[c][0];
-            if (dd_le_d(d, 0.0) || dd_isnan(d)) {
-                bad = 1;
-                *vfail = 1;
-                *info = c0 + j + 1;
-            } else {
-                const dd_t l = dd_sqrt(d);
-                x[c][0] = l;
-                const dd_t r = dd_div(dd_from(1.0), l);
-                if (rdiag) rdiag[j] = r;
-                rh = r.hi;
-                rl = r.lo;
-            }
-        }
-        bad = __shfl_sync(0xffffffffu, bad, 0);
-        if (!bad) {
-            const dd_t r = dd_make(__shfl_sync(0xffffffffu, rh, 0), __shfl_sync(0xffffffffu, rl, 0));
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int i = j + lane + 32 * q;
-                if (i < nb) {
-                    if (i > j) x[c][q] = dd_mul(r, x[c][q]);
-                    S[i + nb * j] = make_double2(x[c][q].hi, x[c][q].lo);
-                }
-            }
-        }
-        mbar_arrive(&bar[j]);
-        return !bad;
-    };
-    // column warp + 32 c takes column k's term
-    auto update = [&](const int c, const int k) {
-        const int j = warp + 32 * c;
-        const double2 l = S[j + nb * k];
-        const dd_t ljk = dd_make(l.x, l.y);
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int i = j + lane + 32 * q;
-            if (i < nb) {
-                const double2 v = S[i + nb * k];
-                x[c][q] = dd_sub(x[c][q], dd_mul(ljk, dd_make(v.x, v.y)));
-            }
-        }
-    };
-    const bool two = warp + 32 < nb;
-    const int last = two ? warp + 32 : (warp < nb ? warp : -1); // the warp's last column
-    bool ok = true;
-    if (warp == 0 && nb > 0) ok = finish(0);
-    for (int k = 0; ok && k < last; ++k) {
-        // warp-uniform outcomes: the lanes go on together or stop together
-        if (!__all_sync(0xffffffffu, bar_wait0(&bar[k]))) {
-            if (lane == 0) {
-                *vfail = 2;
-                atomicCAS(info, 0, -1);
-            }
-            break;
-        }
-        if (__any_sync(0xffffffffu, *vfail != 0)) break;
-        if (((k + 1) & 31) == warp) {
-            // this warp owns column k + 1
-            if (k + 1 < 32) {
-                update(0, k);
-                ok = finish(0);
-                if (ok && two) update(1, k);
-            } else {
-                update(1, k);
-                ok = finish(1);
-            }
-        } else {
-            if (warp > k) update(0, k);
-            if (two) update(1, k);
+    if (tid == 0) stop = 0;
+    for (int e = tid; e < nb * nb; e += DIAG_THREADS) {
+        const int i = e % nb, j = e / nb;
+        if (i >= j) {
+            const dd_t v = ld_dd(A + (c0 + i) + lda * (long)(c0 + j));
+            S[e] = make_double2(v.hi, v.lo);
         }
     }
     __syncthreads();
-    if (*vfail) return;
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int j = warp + 32 * c, i = j + lane + 32 * r;
-            if (j < nb && i < nb) st_dd(A + (c0 + i) + lda * (long)(c0 + j), x[c][r]);
+    volatile int *vstop = &stop;
+    auto at = [&](int i, int j) {
+        const double2 v = S[i + nb * j];
+        return dd_make(v.x, v.y);
+    };
+    auto put = [&](int i, int j, dd_t v) { S[i + nb * j] = make_double2(v.hi, v.lo); };
+    // Named barriers, four of a kind in turn (by k).  Column k published (k <
+    // nb - 2): warp 0 arrives, the helpers wait, so none is a whole turn
+    // behind.  Column k handed over (k >= 2): its helper arrives, warp 0 waits.
+    auto bar_arrive = [](int id, int warps) {
+        __syncwarp();
+        asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(32 * warps) : "memory");
+    };
+    auto bar_wait = [](int id, int warps) {
+        __syncwarp();
+        asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(32 * warps) : "memory");
+    };
+    auto column_id = [](int k) { return 1 + (k & 3); };
+    auto handed_id = [](int k) { return 5 + (k & 3); };
+    const int columns = nb - 2;
+    if (warp == 0) {
+        const int i0 = min(lane, nb - 1), i1 = min(lane + 32, nb - 1); // (a repeated last row is not stored)
+        // column k is c - ln L(:, k - 1)
+        dd_t ca = at(i0, 0), cb = at(i1, 0), ln = dd_zero(), la = ln, lb = ln, d = at(0, 0);
+        for (int k = 0; k < nb; ++k) {
+            if (dd_le_d(d, 0.0) || dd_isnan(d)) {
+                if (lane == 0) {
+                    *info = c0 + k + 1;
+                    *vstop = k + 1; // the helpers stop at column k
+                }
+                if (k < columns) bar_arrive(column_id(k), 1 + DIAG_HELPERS);
+                break;
+            }
+            const int kn = min(k + 1, nb - 1);
+            dd_t l, r;
+            const bool fast = sqrt_rcp_fast(d, l, r);
+            // the column's last term, and its entry of the next row in every
+            // lane, beside the pivot's chain
+            const dd_t ua = dd_sub(ca, dd_mul(ln, la)), ub = dd_sub(cb, dd_mul(ln, lb));
+            const dd_t xa = k > 0 ? ua : ca, xb = k > 0 ? ub : cb;
+            const dd_t xn = shfl_dd(kn < 32 ? xa : xb, kn & 31);
+            if (!fast) sqrt_rcp_plain(d, l, r);
+            if (kn >= 2 && kn > k) bar_wait(handed_id(kn), 2);
+            const dd_t dn = at(kn, kn);
+            ca = at(i0, kn);
+            cb = at(i1, kn);
+            ln = dd_mul(r, xn);
+            d = dd_sub(dn, dd_mul(ln, ln));
+            la = lane == k ? l : dd_mul(r, xa);
+            lb = lane + 32 == k ? l : dd_mul(r, xb);
+            if (lane >= k && lane < nb) put(i0, k, la);
+            if (lane + 32 >= k && lane + 32 < nb) put(i1, k, lb);
+            if (lane == 0 && rdiag) st_dd(rdiag + k, r);
+            if (k < columns) bar_arrive(column_id(k), 1 + DIAG_HELPERS);
         }
+    } else if ((warp & 3) != 0) {
+        const int h = (warp >> 2) * 3 + (warp & 3) - 1;
+        // pair p: columns ja = 2 + p and jb = nb - p (none: -1); slot q of the
+        // lane: entry q 32 + lane of the rows ja .. nb-1 of ja, then jb .. nb-1
+        // of jb
+        dd_t x[DIAG_PAIRS][2];
+        int col[DIAG_PAIRS][2], row[DIAG_PAIRS][2], ja[DIAG_PAIRS], jb[DIAG_PAIRS];
+#pragma unroll
+        for (int c = 0; c < DIAG_PAIRS; ++c) {
+            const int p = h + DIAG_HELPERS * c;
+            ja[c] = 2 + p;
+            jb[c] = nb - p;
+            if (ja[c] > jb[c] || ja[c] >= nb) ja[c] = jb[c] = -1;
+            if (jb[c] == ja[c] || jb[c] >= nb) jb[c] = -1;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int e = q * 32 + lane, na = ja[c] < 0 ? 0 : nb - ja[c];
+                col[c][q] = e < na ? ja[c] : jb[c];
+                row[c][q] = e < na ? ja[c] + e : jb[c] + e - na;
+                if (col[c][q] < 0 || row[c][q] >= nb) col[c][q] = -1, row[c][q] = 0;
+                x[c][q] = col[c][q] >= 0 ? at(row[c][q], col[c][q]) : dd_zero();
+            }
+        }
+        for (int k = 0; k < columns; ++k) {
+            bar_wait(column_id(k), 1 + DIAG_HELPERS);
+            if (*vstop == k + 1) break;
+            auto update = [&](const int c) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int j = col[c][q];
+                    if (!__any_sync(0xffffffffu, j >= k + 2)) continue;
+                    x[c][q] = dd_sub(x[c][q], dd_mul(at(max(j, k), k), at(max(row[c][q], k), k)));
+                    if (j == k + 2) put(row[c][q], j, x[c][q]);
+                }
+                if (ja[c] == k + 2 || jb[c] == k + 2) bar_arrive(handed_id(k + 2), 2);
+            };
+            static_assert(DIAG_PAIRS == 2, "the urgent pair first");
+            if (ja[1] == k + 2 || jb[1] == k + 2) {
+                update(1);
+                update(0);
+            } else {
+                update(0);
+                update(1);
+            }
+        }
+    }
+    __syncthreads();
+    if (stop != 0) return;
+    for (int e = tid; e < nb * nb; e += DIAG_THREADS) {
+        const int i = e % nb, j = e / nb;
+        if (i >= j) st_dd(A + (c0 + i) + lda * (long)(c0 + j), at(i, j));
+    }
 }
 
 // Panel rows below the diagonal block (Rtrsm "Right", "Lower", "Transpose":
@@ -806,9 +837,6 @@ __device__ __forceinline__ void trsv_load_tile(double2 *T, const TrsvArgs &a, in
 __device__ __forceinline__ dd_t ldcg_dd(const dd_t *p) {
     const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
     return dd_make(v.x, v.y);
-}
-__device__ __forceinline__ dd_t shfl_dd(dd_t v, int src) {
-    return dd_make(__shfl_sync(0xffffffffu, v.hi, src), __shfl_sync(0xffffffffu, v.lo, src));
 }
 
 // The diagonal tile by warp 0: entries lane and 32 + lane in v0, v1; steps s
