@@ -764,8 +764,8 @@ void zero_upper(cudaStream_t st, dd_t *A, long lda, int n, int batch, long sA) {
 // A CTA waits for a block with an acquire load bounded by the solve's wait
 // budget (2 s by default); on expiry it records the block in the error word
 // and returns.  Tests of that path name a block whose flag is withheld.
-// Measured, n = 1327: 413 us forward, 409 backward, for one right-hand side
-// or two side by side (20 us a block, 13 of them in its diagonal tile); with
+// Measured, n = 1327: 402 us forward, 400 backward, for one right-hand side
+// or two side by side (19 us a block, 13 of them in its diagonal tile); with
 // one warp that multiplied, subtracted and divided for all 64 entries 747
 // and 622 us each.
 constexpr int TRSV_B = 64;
@@ -865,6 +865,8 @@ template <bool FWD> __device__ __forceinline__ void trsv_diag(const double2 *T, 
     l = el(s1, s1);
     for (int q = 0; q < nb; ++q) {
         const int s2 = at(q + 2);
+        const dd_t ln = el(s2, s2), gn = el(s2, s1), g0 = el(lane, s1), g1 = el(32 + lane, s1);
+        const double yn = rd[s2];
         const bool skip = FWD && dd_is_zero(x);
         const dd_t nv = dd_sub(w, dd_mul(x, fn));
         const dd_t n0 = dd_sub(v0, dd_mul(x, f0)), n1 = dd_sub(v1, dd_mul(x, f1));
@@ -873,8 +875,7 @@ template <bool FWD> __device__ __forceinline__ void trsv_diag(const double2 *T, 
         v0 = lane == s ? x : u0 ? n0 : v0;
         v1 = 32 + lane == s ? x : u1 ? n1 : v1;
         x = fast(w, l, y);
-        const dd_t wn = entry(s2), ln = el(s2, s2), gn = el(s2, s1), g0 = el(lane, s1), g1 = el(32 + lane, s1);
-        const double yn = rd[s2];
+        const dd_t wn = entry(s2);
         if (y == 0.0 || !mid_range(w.hi)) x = plain(w, l);
         w = wn, l = ln, fn = gn, f0 = g0, f1 = g1, y = yn;
         s = s1;
