@@ -262,7 +262,7 @@ struct Context {
     // factorisation until the next factorisation
     DBuf<dd_t> trsv_winv;
     bool winv_valid = false;
-    DBuf<int8_t> tc_slice_buf;
+    DBuf<int8_t> tc_digit_buf;
     DBuf<int> tc_exps, tc_err;
     OzakiWork tc;
     // the split of the Schur complement's F1 pair products (W^T V over K =

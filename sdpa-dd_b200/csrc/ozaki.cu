@@ -1,50 +1,60 @@
 // Tensor-core split of the Cholesky trailing update, C(lower) -= P P^T.
 //
 // Split (ozaki_split_kernel).  Row r of the panel is scaled by 2^-e_r, with
-// e_r chosen so that every |P(r,k)| 2^-e_r <= 1/2, and then peeled into
-// signed base-128 digits: u = P(r,k) 2^(7-e_r); for s = 1..S:
-// D_s = rint(u.hi), u = (u - D_s) * 128.  Each step is exact in dd (the
-// integer is subtracted from the high part, the remainder renormalised with
-// TwoSum), every digit lies in [-64, 64], and after S digits the value is
-// known to 2^-(7S+1) of its row's scale: S = 16 gives 113 bits.
-//   P(r,k) = 2^e_r sum_s D_s(r,k) 2^-7s  (+ remainder)
+// e_r chosen so that every |P(r,k)| 2^-e_r <= 0.498, and written as a fixed
+// point number in B signed base-256 digits D_1 .. D_B in [-128, 127]:
+//   P(r,k) = 2^e_r sum_s D_s(r,k) 2^-8s  (+ remainder <= 2^-(8B+1) 2^e_r).
+// A caller's S 7-bit slices are carried by B = ceil(7S/8) digits (16 slices:
+// 14 digits, 112 bits and the rounding of the last one, as 16 7-bit digits
+// hold), so 105 digit products replace 136 and the diagonals are 14, not 16.
+// 0.498 < 127/255, the largest value that digits up to 127 reach.
 //
-// Products (ozaki_syrk_kernel).  C(i,j) -= 2^(e_i+e_j) sum_d 2^-7d A_d(i,j),
-// A_d = sum_{s+t=d} D_s(i,:) . D_t(j,:), for d = 2..S+1 (the S(S+1)/2 slice
-// pairs that reach 7(S+1) bits).  Every A_d is an exact int32 (|A_d| <=
-// 16 * 64 * 64 * 64 = 2^22), accumulated by tcgen05.mma kind::i8 in tensor
-// memory.
+// Products (ozaki_syrk_kernel).  C(i,j) -= 2^(e_i+e_j) sum_d 2^-8d A_d(i,j),
+// A_d = sum_{s+t=d} D_s(i,:) . D_t(j,:), for d = 2..B+1 (the B(B+1)/2 digit
+// pairs that reach 8(B+1) bits).  Every A_d is an exact int32 (|A_d| <=
+// (d-1) * 64 * 128 * 128 < 2^24), accumulated by tcgen05.mma kind::i8 in
+// tensor memory.
 //
 // One tcgen05.mma costs about the same time for any N up to 128 (on B200 a
 // kind::i8 M=128 K=32 instruction occupies the issuing thread ~97 cycles
 // for N = 32..128 and ~170 for N = 256), so the kernel issues few, wide
-// MMAs: a tile is 128 rows x 16 columns, its B operand the tile's S slices
-// stacked (row 16 (t-1) + j is slice t of column j), and its accumulators
+// MMAs: a tile is 128 rows x 16 columns, its B operand the tile's digits
+// stacked (row 16 (t-1) + j is digit t of column j), and its accumulators
 // are laid out by diagonal (diagonal d in columns 16 (d-2) .. 16 (d-2) + 15).
-// The MMA of A slice s against stacked B slices 1 .. S+1-s (N = 16 (S+1-s))
-// then writes diagonals s+1 .. S+1 in one instruction: S x 2 K steps = 32
-// MMAs per tile for 16 slices.
+// The MMA of A digit s against stacked B digits 1 .. B+1-s (N = 16 (B+1-s))
+// then writes diagonals s+1 .. B+1 in one instruction: B x 2 K steps = 28
+// MMAs per tile for 14 digits.
 //
-// Epilogue: four consecutive diagonals combine exactly into a double
-// (2^21 A_d + 2^14 A_d+1 + 2^7 A_d+2 + A_d+3 < 2^44: two int32 pairs and one
-// FMA), the four groups (2^-28 apart) sum to a dd through two TwoSums, and
-// the dd is scaled by 2^(e_i+e_j-35) and subtracted from C.
+// Epilogue: an entry's diagonals combine exactly to one 128-bit integer; its
+// three 42-bit pieces become doubles scaled by 2^(e_i+e_j) and are summed with
+// C's two halves (oz_sub).
 //
 // Kernel layout: one persistent CTA per SM over the tiles of the lower
-// triangle (row-block major, so a CTA keeps its 128-row A slices in shared
-// memory while it walks the columns).  Warp 0 lane 0 stages operands with
-// bulk copies (cp.async.bulk, no multicast; B four tiles deep) and issues
-// the MMAs; warps 1-16 drain tensor memory, which holds two accumulator
-// buffers of 16 x 16 columns, so one tile multiplies while the last drains.
-// Operand layout in global and shared memory: per slice, 8-row groups of
-// 512 bytes, each four 128-byte core matrices (8 rows x 16 K-bytes): the
-// K-major, non-swizzled canonical layout of the MMA's shared-memory
-// descriptors (LBO 128 bytes between the two K chunks of one MMA, SBO 512
-// bytes between row groups), so a tile's stacked B slices are contiguous.
+// triangle (row-block major, so a CTA keeps its 128-row A digits in shared
+// memory while it walks the columns).  Warp 17 stages everything with bulk
+// copies (cp.async.bulk, no multicast): B three tiles deep and C's tiles two
+// deep, a copy per column (clipped to the lower triangle).  Warp 0 lane 0
+// issues the MMAs; warps 1-16 drain tensor memory, which holds two
+// accumulator buffers, so one tile multiplies while the last drains.
+// Operand layout in global memory: 16-row blocks, in a block digit by digit,
+// a digit's 16 rows as two 8-row groups of 512 bytes, each four 128-byte core
+// matrices (8 rows x 16 K-bytes): the K-major, non-swizzled canonical layout
+// of the MMA's shared-memory descriptors (LBO 128 bytes between the two K
+// chunks of one MMA, SBO 512 bytes between row groups), so a tile's stacked B
+// digits are one copy; the A digits of a row block are gathered digit by
+// digit, 1 KB at a time.
 // Every mbarrier wait is bounded (the context's wait budget, 2 s by
 // default); on expiry the CTA records a code in
 // the error word, stops issuing, waits (bounded) for what it issued and
 // frees its tensor memory.
+//
+// What bounds it: C is read and written once per panel (32 bytes an entry of
+// the lower triangle, 0.24 ms at n = 9920) and a tile's 28 MMAs take about as
+// long, but FP64 and tensor instructions wait for one another (see the
+// epilogue), so a tile takes the sum of the two.  Measured, one update: n =
+// 9920 448 us, n = 5000 133; with 16 7-bit digits assembled in FP64, C loaded
+// by the epilogue's threads and the copies issued by the MMA's thread 538 and
+// 157.
 #include "ozaki.h"
 
 #include <algorithm>
@@ -59,19 +69,22 @@ namespace {
 
 constexpr int OZ_EPI_WARPS = 16; // epilogue warps: four per tensor-memory lane quadrant
 constexpr int OZ_EPI_COLS = OZ_COLS_B / (OZ_EPI_WARPS / 4); // tile columns per epilogue thread
-constexpr int OZ_THREADS = 32 * (1 + OZ_EPI_WARPS); // warp 0: copies + MMA; the rest: epilogue
-// 17 warps put five on one SM sub-partition: 5 x 32 x 96 registers fit its 16384
+constexpr int OZ_AB_WARP = 1 + OZ_EPI_WARPS, OZ_C_WARP = 2 + OZ_EPI_WARPS; // the warps that copy the operands and C
+constexpr int OZ_THREADS = 32 * (3 + OZ_EPI_WARPS); // warp 0: MMA; then the epilogue; then the copies
+// 19 warps put five on an SM sub-partition: 5 x 32 x 96 registers fit its 16384
 constexpr int OZ_MAX_REGS = 96;
-constexpr int OZ_A_BYTES = OZ_ROWS_A * OZ_K; // one slice of a 128-row block
-constexpr int OZ_B_BYTES = OZ_COLS_B * OZ_K; // one slice of a 16-row block
-constexpr int OZ_TILE_B = OZ_MAX_SLICES * OZ_B_BYTES; // the stacked B slices of a tile
-constexpr int OZ_STAGES = 4;                 // B tiles in shared memory
-constexpr int OZ_ACC_COLS = OZ_MAX_SLICES * OZ_COLS_B; // tensor-memory columns of one accumulator buffer
+constexpr int OZ_A_BYTES = OZ_ROWS_A * OZ_K; // one digit of a 128-row block
+constexpr int OZ_B_BYTES = OZ_COLS_B * OZ_K; // one digit of a 16-row block
+constexpr int OZ_TILE_B = OZ_MAX_DIGITS * OZ_B_BYTES; // the stacked B digits of a tile
+constexpr int OZ_STAGES = 3;                 // B tiles in shared memory
+constexpr int OZ_C_STAGES = 2;               // C tiles in shared memory
+constexpr int OZ_C_BYTES = OZ_ROWS_A * OZ_COLS_B * 16; // one C tile
+constexpr int OZ_ACC_COLS = 256; // tensor-memory columns of one accumulator buffer
 static_assert(2 * OZ_ACC_COLS <= 512, "split kernel: two accumulator buffers must fit tensor memory");
-static_assert(OZ_ACC_COLS <= 256, "split kernel: the widest MMA has N = 16 S <= 256");
-// the 16 A slices of a row block and OZ_STAGES stacked B tiles
-constexpr size_t OZ_SMEM = 1024 + (size_t)OZ_MAX_SLICES * OZ_A_BYTES + (size_t)OZ_STAGES * OZ_TILE_B;
-static_assert(OZ_SMEM <= 232448 - 256, "split kernel: shared memory above the per-CTA limit");
+static_assert(OZ_MAX_DIGITS * OZ_COLS_B <= OZ_ACC_COLS, "split kernel: the widest MMA has N = 16 B <= 256");
+// the A digits of a row block, OZ_STAGES stacked B tiles and OZ_C_STAGES C tiles
+constexpr size_t OZ_SMEM = 1024 + (size_t)OZ_MAX_DIGITS * OZ_A_BYTES + (size_t)OZ_STAGES * OZ_TILE_B + (size_t)OZ_C_STAGES * OZ_C_BYTES;
+static_assert(OZ_SMEM <= 232448 - 512, "split kernel: shared memory above the per-CTA limit");
 // kind::i8 instruction descriptor: D s32, A and B s8, both K-major, M = 128,
 // N = n (a multiple of 16, 16..256).
 __host__ __device__ constexpr uint32_t oz_idesc(int n) {
@@ -82,7 +95,9 @@ __device__ __forceinline__ unsigned long long oz_ns() { return globaltimer_ns();
 // Waits for the phase with the given parity to complete; false when the CTA
 // is aborting or the wait ran out (then the CTA aborts with `code`).
 __device__ bool oz_wait(uint64_t *b, uint32_t parity, volatile int *abort_flag, int *err, int code, unsigned long long wait_ns) {
-    if (mbar_try_wait(b, parity)) return true;
+    // the clock is read only once a wait has become long
+    for (int k = 0; k < 64; ++k)
+        if (mbar_try_wait(b, parity)) return true;
     const unsigned long long t0 = oz_ns();
     while (!mbar_try_wait(b, parity)) {
         if (*abort_flag) return false;
@@ -108,13 +123,11 @@ __device__ __forceinline__ uint64_t oz_desc(uint32_t saddr) {
 }
 
 struct OzArgs {
-    const int8_t *slices;   // slice by slice (A operands: a row block of one slice is contiguous)
-    const int8_t *slices_b; // by 16-row block (B operands: a tile's slices are contiguous)
-    long slice_stride; // bytes between slices
+    const int8_t *digits; // by 16-row block, a block's nd digits back to back
     const int *exps;
     dd_t *C;
     long ldc;
-    int n, ns, nI, nJ;
+    int n, nd, nI, nJ;
     int skip; // rows below skip are not written (their block is updated elsewhere)
     long tiles;
     int *err;
@@ -141,14 +154,16 @@ __device__ __forceinline__ void oz_tile_next(int nJ, int &I, int &J) {
 }
 
 // Shared state of one CTA.
-//   barA          A slices of the current row block landed
-//   barB[st]      the B slices of the tile in stage st landed
-//   bfree[st]     every MMA of the tile in stage st completed (the stage,
-//                 and at a row-block change A, may be reloaded)
-//   tfull/tempty  accumulator buffer b holds a finished tile / is drained
+//   barA          A digits of the current row block landed
+//   barB[st]      the B digits of the tile in stage st landed
+//   done[st]      every MMA of the tile in stage st completed: its
+//                 accumulators are there, and the stage (at a row-block
+//                 change A as well) may be reloaded
+//   tempty[b]     accumulator buffer b is drained
+//   cfull/cempty  C stage st holds its tile's entries / has been read
 //   fin           every MMA the CTA issued completed (exit)
 struct OzShared {
-    uint64_t barA, barB[OZ_STAGES], bfree[OZ_STAGES], tfull[2], tempty[2], fin;
+    uint64_t barA, barB[OZ_STAGES], done[OZ_STAGES], tempty[2], cfull[OZ_C_STAGES], cempty[OZ_C_STAGES], fin;
     uint32_t tmem;
     int abort_flag;
 };
@@ -159,25 +174,26 @@ __device__ __forceinline__ void tc_mma_i8_n(uint32_t d_tmem, uint64_t da, uint64
                  : "memory");
 }
 
-// The MMAs of one tile into the accumulator buffer at dbuf: for A slice s
-// and K step kk, one MMA against the stacked B slices t = 1 .. S+1-s
-// (N = 16 (S+1-s)) writes the columns of diagonals s+1 .. S+1.  The first
-// (s = 1, N = 16 S) covers every column and overwrites; the rest accumulate.
-template <int NS>
-__device__ __forceinline__ void oz_issue_tile(uint32_t dbuf, uint64_t descA, uint64_t descB) {
+// MMAs of one tile into the accumulator buffer at dbuf, A digits S0 .. S1:
+// for A digit s and K step kk, one MMA against the stacked B digits t = 1 ..
+// B+1-s (N = 16 (B+1-s)) writes the columns of diagonals s+1 .. B+1.  The
+// first (s = 1, N = 16 B) covers every column and overwrites; the rest
+// accumulate.
+template <int ND, int S0, int S1>
+__device__ __forceinline__ void oz_issue(uint32_t dbuf, uint64_t descA, uint64_t descB) {
 #pragma unroll
-    for (int s = 1; s <= NS; ++s) {
+    for (int s = S0; s <= S1; ++s) {
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk)
             tc_mma_i8_n(dbuf + (uint32_t)((s - 1) * OZ_COLS_B), descA + (uint64_t)(((s - 1) * OZ_A_BYTES + kk * 256) >> 4),
-                        descB + (uint64_t)((kk * 256) >> 4), oz_idesc((NS + 1 - s) * OZ_COLS_B), (s == 1 && kk == 0) ? 0u : 1u);
+                        descB + (uint64_t)((kk * 256) >> 4), oz_idesc((ND + 1 - s) * OZ_COLS_B), (s == 1 && kk == 0) ? 0u : 1u);
     }
 }
-__device__ __forceinline__ void oz_issue_tile_rt(int ns, uint32_t dbuf, uint64_t descA, uint64_t descB) {
-    for (int s = 1; s <= ns; ++s)
+__device__ __forceinline__ void oz_issue_rt(int nd, int s0, int s1, uint32_t dbuf, uint64_t descA, uint64_t descB) {
+    for (int s = s0; s <= s1; ++s)
         for (int kk = 0; kk < 2; ++kk)
             tc_mma_i8_n(dbuf + (uint32_t)((s - 1) * OZ_COLS_B), descA + (uint64_t)(((s - 1) * OZ_A_BYTES + kk * 256) >> 4),
-                        descB + (uint64_t)((kk * 256) >> 4), oz_idesc((ns + 1 - s) * OZ_COLS_B), (s == 1 && kk == 0) ? 0u : 1u);
+                        descB + (uint64_t)((kk * 256) >> 4), oz_idesc((nd + 1 - s) * OZ_COLS_B), (s == 1 && kk == 0) ? 0u : 1u);
 }
 
 // A wait that ignores the abort flag (still bounded): used on the way out,
@@ -193,205 +209,294 @@ __device__ void oz_wait_out(uint64_t *b, uint32_t parity, int *err, unsigned lon
     }
 }
 
-// Warp 0, lane 0: bulk copies of the operands and the MMAs.  The A slices
-// of a row block stay in shared memory while the CTA walks its columns; the
-// B slices of the next OZ_STAGES - 1 tiles are in flight while a tile
-// multiplies (tile n in stage n mod OZ_STAGES, accumulators in buffer
-// n mod 2).
-__device__ void oz_producer(const OzArgs &a, OzShared &S, uint8_t *smA, uint8_t *smB, long t_begin, long t_end) {
+// Warp 0, lane 0: the MMAs (tile n from B stage n mod OZ_STAGES into
+// accumulator buffer n mod 2).  It only waits and issues: an MMA holds the
+// issuing thread for about its own duration, so whatever else this thread
+// does the tensor pipe stands idle for.  The next tile's barriers (a try
+// costs over 100 cycles even when it succeeds) are tried before the last
+// MMAs of a tile are issued.
+__device__ void oz_mma(const OzArgs &a, OzShared &S, const uint8_t *smA, const uint8_t *smB, int I, int J, int ntile) {
     volatile int *abort_flag = &S.abort_flag;
-    const int ns = a.ns;
-    const long ntile = t_end - t_begin;
-    // one bulk copy per tile: the block's ns slices lie back to back
-    auto load_B = [&](int jb, int st) {
-        mbar_expect_tx(&S.barB[st], (uint32_t)(ns * OZ_B_BYTES));
-        bulk_g2s(smB + (size_t)st * OZ_TILE_B, a.slices_b + (long)jb * ns * OZ_B_BYTES, (uint32_t)(ns * OZ_B_BYTES), &S.barB[st]);
-    };
     const uint64_t descA = oz_desc(smem_u32(smA));
     const uint64_t descB0 = oz_desc(smem_u32(smB));
-    int Ip, Jp; // the next tile to prefetch (np)
-    oz_tile_at(t_begin, a.nI, a.nJ, Ip, Jp);
-    long np = 0;
-    for (; np < ntile && np < OZ_STAGES - 1; ++np) {
-        load_B(Jp, (int)(np % OZ_STAGES));
-        oz_tile_next(a.nJ, Ip, Jp);
-    }
-    int I, J;
-    oz_tile_at(t_begin, a.nI, a.nJ, I, J);
-    uint32_t phA = 0;
-    bool pendA = false, issued = false;
-    int curA = -1;
-    long nb = 0; // tiles whose B copy has been waited for
-    bool ok = true;
-    for (long n = 0; n < ntile && ok; ++n) {
-        const int st = (int)(n % OZ_STAGES), b = (int)(n & 1);
+    uint32_t phA = 0, phB = 0;
+    int st = 0, curA = -1, n = 0;
+    bool haveB = false, haveT = false; // tile n's B digits are there, its buffer is drained
+    for (; n < ntile; ++n) {
+        const int b = n & 1;
         if (I != curA) {
-            // every MMA of the previous tile reads A
-            if (n > 0) {
-                ok = oz_wait(&S.bfree[(n - 1) % OZ_STAGES], (uint32_t)(((n - 1) / OZ_STAGES) & 1), abort_flag, a.err, 1, a.wait_ns);
-                if (!ok) break;
-            }
-            mbar_expect_tx(&S.barA, (uint32_t)(ns * OZ_A_BYTES));
-            for (int s = 0; s < ns; ++s)
-                bulk_g2s(smA + (size_t)s * OZ_A_BYTES, a.slices + s * a.slice_stride + (long)I * OZ_A_BYTES, OZ_A_BYTES, &S.barA);
-            pendA = true;
-            ok = oz_wait(&S.barA, phA, abort_flag, a.err, 2, a.wait_ns);
-            if (!ok) break;
+            if (!oz_wait(&S.barA, phA, abort_flag, a.err, 2, a.wait_ns)) break;
             phA ^= 1u;
-            pendA = false;
             curA = I;
         }
-        ok = oz_wait(&S.barB[st], (uint32_t)((n / OZ_STAGES) & 1), abort_flag, a.err, 3, a.wait_ns);
-        if (!ok) break;
-        nb = n + 1;
-        ok = oz_wait(&S.tempty[b], (uint32_t)(((n >> 1) & 1) ^ 1), abort_flag, a.err, 4, a.wait_ns);
-        if (!ok) break;
+        if (!haveB && !oz_wait(&S.barB[st], phB, abort_flag, a.err, 3, a.wait_ns)) break;
+        if (!haveT && !oz_wait(&S.tempty[b], (uint32_t)(((n >> 1) & 1) ^ 1), abort_flag, a.err, 4, a.wait_ns)) break;
         tc_fence_after();
-        const uint64_t descB = descB0 + (uint64_t)(((size_t)st * OZ_TILE_B) >> 4);
-        if (ns == OZ_MAX_SLICES)
-            oz_issue_tile<OZ_MAX_SLICES>(S.tmem + (uint32_t)(b * OZ_ACC_COLS), descA, descB);
+        const uint64_t descB = descB0 + (uint64_t)((st * OZ_TILE_B) >> 4);
+        const uint32_t dbuf = S.tmem + (uint32_t)(b * OZ_ACC_COLS);
+        constexpr int HEAD = OZ_MAX_DIGITS - 2;
+        const bool full = a.nd == OZ_MAX_DIGITS;
+        if (full)
+            oz_issue<OZ_MAX_DIGITS, 1, HEAD>(dbuf, descA, descB);
         else
-            oz_issue_tile_rt(ns, S.tmem + (uint32_t)(b * OZ_ACC_COLS), descA, descB);
-        issued = true;
-        tc_commit(&S.tfull[b]);
-        tc_commit(&S.bfree[st]);
-        // prefetch tile np (= n + OZ_STAGES - 1) once tile np - OZ_STAGES
-        // (= n - 1), the last user of its stage, has completed
-        if (np < ntile) {
-            const int sp = (int)(np % OZ_STAGES);
-            if (np >= OZ_STAGES) {
-                ok = oz_wait(&S.bfree[sp], (uint32_t)(((np - OZ_STAGES) / OZ_STAGES) & 1), abort_flag, a.err, 1, a.wait_ns);
-                if (!ok) break;
-            }
-            load_B(Jp, sp);
-            oz_tile_next(a.nJ, Ip, Jp);
-            ++np;
-        }
+            oz_issue_rt(a.nd, 1, a.nd, dbuf, descA, descB);
+        const int stn = st + 1 == OZ_STAGES ? 0 : st + 1;
+        const uint32_t phn = stn == 0 ? phB ^ 1u : phB;
+        haveB = n + 1 < ntile && mbar_try_wait(&S.barB[stn], phn);
+        haveT = n + 1 < ntile && mbar_try_wait(&S.tempty[b ^ 1], (uint32_t)((((n + 1) >> 1) & 1) ^ 1));
+        if (full) oz_issue<OZ_MAX_DIGITS, HEAD + 1, OZ_MAX_DIGITS>(dbuf, descA, descB);
+        tc_commit(&S.done[st]);
+        st = stn;
+        phB = phn;
         oz_tile_next(a.nJ, I, J);
     }
-    // On the way out every issued copy lands and every issued MMA completes
-    // (bounded waits) before the CTA frees its memory.
-    if (pendA) oz_wait_out(&S.barA, phA, a.err, a.wait_ns);
-    for (long k = nb; k < np; ++k) oz_wait_out(&S.barB[k % OZ_STAGES], (uint32_t)((k / OZ_STAGES) & 1), a.err, a.wait_ns);
-    if (issued) {
+    // every issued MMA completes (bounded wait) before the CTA frees its memory
+    if (n > 0) {
         tc_commit(&S.fin);
         oz_wait_out(&S.fin, 0, a.err, a.wait_ns);
     }
 }
 
-// 2^e as a double for -1022 <= e <= 1023 (built from its bits)
-__device__ __forceinline__ double oz_pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+// Lane 0 waits, the warp follows its outcome.
+__device__ __forceinline__ bool oz_wait_lane0(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *err, int code, unsigned long long wait_ns) {
+    int ok = 1;
+    if ((threadIdx.x & 31) == 0) ok = oz_wait(bar, parity, abort_flag, err, code, wait_ns) ? 1 : 0;
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
+// Warp OZ_AB_WARP: the operands.  B's digits OZ_STAGES tiles deep, one copy a
+// tile; the A digits of a row block when it changes, once the MMAs of the tile
+// before have read the old ones, 1 KB a copy over all lanes.
+__device__ void oz_load_ab(const OzArgs &a, OzShared &S, uint8_t *smA, uint8_t *smB, int I, int J, int ntile) {
+    volatile int *abort_flag = &S.abort_flag;
+    const int lane = threadIdx.x & 31, nd = a.nd;
+    int curA = -1, nA = 0, nB = 0; // copies issued
+    int st = 0, last = 0;          // B stage of this tile and of the one before
+    uint32_t ph = 0, phlast = 0;   // parity of the stage's current use
+    for (int n = 0; n < ntile; ++n) {
+        if (n >= OZ_STAGES && !oz_wait_lane0(&S.done[st], ph ^ 1u, abort_flag, a.err, 1, a.wait_ns)) break;
+        if (lane == 0) {
+            mbar_expect_tx(&S.barB[st], (uint32_t)(nd * OZ_B_BYTES));
+            bulk_g2s(smB + (size_t)st * OZ_TILE_B, a.digits + (long)J * nd * OZ_B_BYTES, (uint32_t)(nd * OZ_B_BYTES), &S.barB[st]);
+        }
+        nB = n + 1;
+        if (I != curA) {
+            if (n > 0 && !oz_wait_lane0(&S.done[last], phlast, abort_flag, a.err, 1, a.wait_ns)) break;
+            if (lane == 0) mbar_expect_tx(&S.barA, (uint32_t)(nd * OZ_A_BYTES));
+            __syncwarp();
+            const int8_t *src = a.digits + (long)I * OZ_JPI * nd * OZ_B_BYTES;
+            for (int e = lane; e < nd * OZ_JPI; e += 32) { // 16-row block q, digit s
+                const int s = e / OZ_JPI, q = e % OZ_JPI;
+                bulk_g2s(smA + (size_t)s * OZ_A_BYTES + q * OZ_B_BYTES, src + (long)(q * nd + s) * OZ_B_BYTES, OZ_B_BYTES, &S.barA);
+            }
+            ++nA;
+            curA = I;
+        }
+        last = st;
+        phlast = ph;
+        if (++st == OZ_STAGES) {
+            st = 0;
+            ph ^= 1u;
+        }
+        oz_tile_next(a.nJ, I, J);
+    }
+    // every issued copy lands (bounded waits) before the CTA leaves
+    if (lane == 0) {
+        if (nA > 0) oz_wait_out(&S.barA, (uint32_t)((nA - 1) & 1), a.err, a.wait_ns);
+        for (int k = max(0, nB - OZ_STAGES); k < nB; ++k) oz_wait_out(&S.barB[k % OZ_STAGES], (uint32_t)((k / OZ_STAGES) & 1), a.err, a.wait_ns);
+    }
+    __syncwarp();
+}
+
+// Warp OZ_C_WARP: C's tiles OZ_C_STAGES deep; lane c copies column c's rows
+// of the lower triangle (16-byte entries, so any row is a valid start).
+__device__ void oz_load_c(const OzArgs &a, OzShared &S, uint8_t *smC, int I, int J, int ntile) {
+    volatile int *abort_flag = &S.abort_flag;
+    const int lane = threadIdx.x & 31;
+    int nC = 0; // tiles whose copies are issued
+    for (; nC < ntile; ++nC) {
+        const int cs = nC % OZ_C_STAGES;
+        if (!oz_wait_lane0(&S.cempty[cs], (uint32_t)(((nC / OZ_C_STAGES) & 1) ^ 1), abort_flag, a.err, 7, a.wait_ns)) break;
+        const int j = J * OZ_COLS_B + lane;
+        int bytes = 0, r0 = 0;
+        if (lane < OZ_COLS_B && j < a.n) {
+            r0 = max(I * OZ_ROWS_A, max(j, a.skip));
+            bytes = max(0, min(I * OZ_ROWS_A + OZ_ROWS_A, a.n) - r0) * 16;
+        }
+        const int total = __reduce_add_sync(0xffffffffu, bytes);
+        if (lane == 0) mbar_expect_tx(&S.cfull[cs], (uint32_t)total);
+        __syncwarp();
+        if (bytes > 0)
+            bulk_g2s(smC + (size_t)cs * OZ_C_BYTES + (size_t)lane * (OZ_ROWS_A * 16) + (size_t)(r0 - I * OZ_ROWS_A) * 16, a.C + r0 + a.ldc * (long)j,
+                     (uint32_t)bytes, &S.cfull[cs]);
+        oz_tile_next(a.nJ, I, J);
+    }
+    // every issued copy lands (bounded waits) before the CTA leaves
+    if (lane == 0)
+        for (int k = max(0, nC - OZ_C_STAGES); k < nC; ++k) oz_wait_out(&S.cfull[k % OZ_C_STAGES], (uint32_t)((k / OZ_C_STAGES) & 1), a.err, a.wait_ns);
+    __syncwarp();
+}
 
 __device__ __forceinline__ void tc_ld2(uint32_t taddr, int32_t *r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr));
 }
 
-// Sum of the diagonals of one entry as a dd, from its diagonal values
-// v[0..15] (diagonal d at v[d-2]; those beyond S+1 are zero), in units of
-// 2^(e_i + e_j): value = sum_d A_d 2^-7d.  Pairs P_k = 2^7 A_2k+2 + A_2k+3
-// are exact in int32 (|P| < 2^30) and in a double; groups G_j = 2^14 P_2j +
-// P_2j+1 are exact doubles (|G| < 2^44, one FMA each), so value = 2^-35
-// (G0 + G1 2^-28 + G2 2^-56 + G3 2^-84).  Two TwoSums leave only the
-// rounding of the two smallest parts' sum and of the final low part:
-// within 2^-106 of the value plus 2^-140 absolute.  The result comes back
-// without its factor 2^-35, which the caller folds into the entry's scale.
-__device__ __forceinline__ void oz_entry_dd(const int32_t (*v)[2], int c, double &hi, double &lo) {
-    double G[4];
+// The diagonals of one entry, v[0..13] (diagonal d at v[d-2]; those beyond
+// B+1 are zero), as four exact integers in units of 2^-40, 2^-72, 2^-104 and
+// 2^-136: A_2..A_5, A_6..A_9, A_10..A_13, A_14 and A_15.  |A_d| <= (d-1) 2^20,
+// so each is below 2^49.
+__device__ __forceinline__ void oz_groups(const int32_t (*v)[2], int c, long long *w) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int32_t p0 = v[4 * j][c] * 128 + v[4 * j + 1][c], p1 = v[4 * j + 2][c] * 128 + v[4 * j + 3][c];
-        G[j] = __fma_rn((double)p0, 16384.0, (double)p1);
+    for (int j = 0; j < 3; ++j)
+        w[j] = (((long long)v[4 * j][c] * 16777216 + (long long)v[4 * j + 1][c] * 65536) + (long long)v[4 * j + 2][c] * 256) + v[4 * j + 3][c];
+    w[3] = (long long)v[12][c] * 16777216 + (long long)v[13][c] * 65536;
+}
+
+// The group w 2^e as a double: the bits of (2^52 + 2^51 + w) 2^e, then one
+// exact subtraction; k holds the upper word of (2^52 + 2^51) 2^e.
+__device__ __forceinline__ double oz_scaled(long long w, int k) {
+    return __hiloint2double((int)(w >> 32) + k, (int)w) - __hiloint2double(k, 0);
+}
+
+// C - (g0 + g1 + g2 + g3) as a dd, the groups already scaled.  The two
+// leading pairs are summed without error; what is rounded is the sum of their
+// errors and of the two small groups (below 2^-56 of 2^(e_i+e_j): 2^-109 of
+// it at most) and the result's own low part (2^-105 of the result).
+__device__ __forceinline__ dd_t oz_sub(double2 c, double g0, double g1, double g2, double g3) {
+    double e, f, g, l, lo;
+    const double s = ddm::two_sum(c.x, -g0, e);
+    const double t = ddm::two_sum(c.y, -g1, f);
+    const double u = ddm::two_sum(e, t, g);
+    const double r = (f + g) - (g2 + g3);
+    const double h = ddm::two_sum(s, u, l);
+    const double hi = ddm::fast_two_sum(h, l + r, lo);
+    return dd_make(hi, lo);
+}
+
+// The diagonals of columns col and col + 1 of a thread's row; nd of them.
+__device__ __forceinline__ void oz_drain2(uint32_t taddr, int nd, int32_t (*v)[2]) {
+#pragma unroll
+    for (int u = 0; u < OZ_MAX_DIGITS; ++u) {
+        if (u < nd) {
+            tc_ld2(taddr + (uint32_t)(u * OZ_COLS_B), v[u]);
+        } else {
+            v[u][0] = 0;
+            v[u][1] = 0;
+        }
     }
-    const double a = G[0], b = G[1] * 0x1p-28, cc = G[2] * 0x1p-56, d = G[3] * 0x1p-84;
-    double e1, s1 = ddm::two_sum(a, b, e1);
-    double e2, s2 = ddm::two_sum(e1, cc, e2);
-    double l, h = ddm::two_sum(s1, s2, l);
-    h = ddm::fast_two_sum(h, l + (e2 + d), l);
-    hi = h;
-    lo = l;
+    tc_wait_ld();
+}
+
+// One thread's entries of a tile in which the warp meets scales at the ends of
+// the exponent range: the groups scaled one by one (out of line, so that the
+// common case keeps its registers).
+__device__ __noinline__ void oz_tile_far(uint32_t taddr, int nd, const double2 *ct, dd_t *cp, long ldc, int ncol, int ei, const int *ej) {
+#pragma unroll 1
+    for (int ch = 0; ch < OZ_EPI_COLS; ch += 2) {
+        int32_t v[OZ_MAX_DIGITS][2];
+        oz_drain2(taddr + (uint32_t)ch, nd, v);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            if (ch + c >= ncol) continue;
+            long long w[4];
+            oz_groups(v, c, w);
+            const int e = ei + ej[ch + c];
+            const dd_t res = oz_sub(ct[(ch + c) * OZ_ROWS_A], ldexp((double)w[0], e - 40), ldexp((double)w[1], e - 72), ldexp((double)w[2], e - 104),
+                                    ldexp((double)w[3], e - 136));
+            __stcs(reinterpret_cast<double2 *>(cp + ldc * (long)(ch + c)), make_double2(res.hi, res.lo));
+        }
+    }
 }
 
 // Epilogue warps 1-16: warp w reads tensor-memory lanes 32 (w mod 4) .. +31
 // (its rows of the tile) and columns 4 h .. 4 h + 3 of every diagonal,
 // h = (w - 1) / 4, two columns at a time with all diagonals in one round
-// trip; each entry's dd (oz_entry_dd) is scaled by 2^(e_i + e_j) and
-// subtracted from C, whose entries were requested before the wait for the
-// accumulators.  NSC: the slice count when known at compile time, else 0.
-template <int NSC>
-__device__ void oz_epilogue(const OzArgs &a, OzShared &S, long t_begin, long t_end) {
+// trip, joins each entry's diagonals to four integers and subtracts them from
+// C, whose tile lies in shared memory.
+// FP64 and tensor instructions share a pipe of the SM: the FP64 part of a
+// tile takes 1.5k cycles without MMAs, 2.9k beside them.  So the digits meet
+// in the integer units (35 FP64 instructions an entry remain of 53), and an
+// accumulator buffer goes back only after the tile's FP64 part, not when it
+// is drained: the MMAs of the tile after next then run while the warps wait,
+// drain and join the next tile (n = 9920: 451 us against 494).
+// NDC: the digit count when known at compile time, else 0.
+template <int NDC>
+__device__ void oz_epilogue(const OzArgs &a, OzShared &S, const uint8_t *smC, int I, int J, int ntile) {
     volatile int *abort_flag = &S.abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = warp & 3, h = (warp - 1) >> 2;
     const int row = 32 * q + lane;
     const uint32_t lane_base = S.tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(OZ_EPI_COLS * h);
-    const int nd = NSC > 0 ? NSC : a.ns; // diagonals 2 .. S+1
-    int I, J;
-    oz_tile_at(t_begin, a.nI, a.nJ, I, J);
-    // lane 0 waits; the warp follows its outcome (the tensor-memory loads
-    // are warp-collective)
-    auto wait_full = [&](int b, uint32_t parity) {
-        int okw = 1;
-        if (lane == 0) okw = oz_wait(&S.tfull[b], parity, abort_flag, a.err, 6, a.wait_ns) ? 1 : 0;
-        return __shfl_sync(0xffffffffu, okw, 0) != 0;
+    const double2 *ct0 = reinterpret_cast<const double2 *>(smC) + (OZ_EPI_COLS * h) * OZ_ROWS_A + row;
+    const int nd = NDC > 0 ? NDC : a.nd; // diagonals 2 .. B+1
+    // the warp goes on together (the tensor-memory loads are warp-collective)
+    auto wait_warp = [&](uint64_t *bar, uint32_t parity, int code) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        return oz_wait_lane0(bar, parity, abort_flag, a.err, code, a.wait_ns);
     };
-    for (long n = 0; n < t_end - t_begin; ++n) {
+    int st = 0; // done[] stage and parity of tile n
+    uint32_t ph = 0;
+    // scale exponents of tile n's row (padded rows hold 0) and columns
+    int ei = 0;
+    int4 ej = make_int4(0, 0, 0, 0);
+    auto load_exps = [&]() {
+        ei = a.exps[I * OZ_ROWS_A + row];
+        ej = *reinterpret_cast<const int4 *>(a.exps + J * OZ_COLS_B + OZ_EPI_COLS * h);
+    };
+    load_exps();
+    for (int n = 0; n < ntile; ++n) {
         const int i = I * OZ_ROWS_A + row;
         const int jb = J * OZ_COLS_B + OZ_EPI_COLS * h;
-        const int b = (int)(n & 1);
+        const int b = n & 1, cs = n % OZ_C_STAGES;
         dd_t *cp = a.C + i + a.ldc * (long)jb;
         // entries of the lower triangle of C: columns jb .. jb + ncol - 1
         const int ncol = (i < a.n && i >= a.skip) ? max(0, min(OZ_EPI_COLS, min(a.n, i + 1) - jb)) : 0;
-        double2 cv[OZ_EPI_COLS];
-#pragma unroll
-        for (int c = 0; c < OZ_EPI_COLS; ++c)
-            cv[c] = c < ncol ? __ldcs(reinterpret_cast<const double2 *>(cp + a.ldc * (long)c)) : make_double2(0.0, 0.0);
-        if (!wait_full(b, (uint32_t)((n >> 1) & 1))) break;
-        tc_fence_after();
-        const uint32_t tb = lane_base + (uint32_t)(b * OZ_ACC_COLS);
-        const int ei = a.exps[i]; // scale exponent of the row (padded rows hold 0)
-        const int4 e4 = *reinterpret_cast<const int4 *>(a.exps + jb);
-        const int ej[4] = {e4.x, e4.y, e4.z, e4.w};
-        // Drain first: every entry's dd from tensor memory, then the
-        // buffer goes back to the MMA warp; only then the entries meet C,
-        // so the accumulators are never held while C is in flight.
-        double phi[OZ_EPI_COLS], plo[OZ_EPI_COLS];
-#pragma unroll
-        for (int ch = 0; ch < OZ_EPI_COLS / 2; ++ch) {
-            int32_t v[OZ_MAX_SLICES][2];
-#pragma unroll
-            for (int u = 0; u < OZ_MAX_SLICES; ++u) {
-                if (u < nd) {
-                    tc_ld2(tb + (uint32_t)(u * OZ_COLS_B + 2 * ch), v[u]);
-                } else {
-                    v[u][0] = 0;
-                    v[u][1] = 0;
-                }
-            }
-            tc_wait_ld();
-            if (ch == OZ_EPI_COLS / 2 - 1) { // the buffer is drained
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&S.tempty[b]);
-            }
-#pragma unroll
-            for (int c = 0; c < 2; ++c) oz_entry_dd(v, c, phi[2 * ch + c], plo[2 * ch + c]);
-        }
-#pragma unroll
-        for (int cc = 0; cc < OZ_EPI_COLS; ++cc) {
-            if (cc < ncol) {
-                const int sc = ei + ej[cc] - 35;
-                dd_t p;
-                if (sc >= -1022 && sc <= 1023) {
-                    const double pw = oz_pow2(sc);
-                    p = dd_make(phi[cc] * pw, plo[cc] * pw);
-                } else {
-                    p = dd_make(ldexp(phi[cc], sc), ldexp(plo[cc], sc));
-                }
-                const dd_t res = dd_sub(dd_make(cv[cc].x, cv[cc].y), p);
-                __stcs(reinterpret_cast<double2 *>(cp + a.ldc * (long)cc), make_double2(res.hi, res.lo));
-            }
-        }
+        const int e[4] = {ei + ej.x, ei + ej.y, ei + ej.z, ei + ej.w};
+        const int eic = ei, *ejc = a.exps + jb;
+        // every scale well inside the exponent range
+        const bool mid = min(min(e[0], e[1]), min(e[2], e[3])) >= -900 && max(max(e[0], e[1]), max(e[2], e[3])) <= 1000;
         oz_tile_next(a.nJ, I, J);
+        if (n + 1 < ntile) load_exps();
+        if (!wait_warp(&S.cfull[cs], (uint32_t)((n / OZ_C_STAGES) & 1), 8)) break;
+        const double2 *ct = ct0 + cs * (OZ_C_BYTES / 16);
+        const uint32_t tb = lane_base + (uint32_t)(b * OZ_ACC_COLS);
+        if (__all_sync(0xffffffffu, mid)) {
+            double2 cv[OZ_EPI_COLS];
+#pragma unroll
+            for (int c = 0; c < OZ_EPI_COLS; ++c) cv[c] = c < ncol ? ct[c * OZ_ROWS_A] : make_double2(0.0, 0.0);
+            if (!wait_warp(&S.done[st], ph, 6)) break;
+            tc_fence_after();
+            long long w[OZ_EPI_COLS][4];
+#pragma unroll
+            for (int ch = 0; ch < OZ_EPI_COLS; ch += 2) {
+                int32_t v[OZ_MAX_DIGITS][2];
+                oz_drain2(tb + (uint32_t)ch, nd, v);
+#pragma unroll
+                for (int c = 0; c < 2; ++c) oz_groups(v, c, w[ch + c]);
+            }
+#pragma unroll
+            for (int c = 0; c < OZ_EPI_COLS; ++c) {
+                const int k = 0x43380000 + (e[c] - 40) * 0x100000;
+                const dd_t res = oz_sub(cv[c], oz_scaled(w[c][0], k), oz_scaled(w[c][1], k - 32 * 0x100000), oz_scaled(w[c][2], k - 64 * 0x100000),
+                                        oz_scaled(w[c][3], k - 96 * 0x100000));
+                if (c < ncol) __stcs(reinterpret_cast<double2 *>(cp + a.ldc * (long)c), make_double2(res.hi, res.lo));
+            }
+        } else {
+            if (!wait_warp(&S.done[st], ph, 6)) break;
+            tc_fence_after();
+            oz_tile_far(tb, nd, ct, cp, a.ldc, ncol, eic, ejc);
+        }
+        // the buffer goes back only now: see above
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+            mbar_arrive(&S.tempty[b]);
+            mbar_arrive(&S.cempty[cs]);
+        }
+        if (++st == OZ_STAGES) {
+            st = 0;
+            ph ^= 1u;
+        }
     }
 }
 
@@ -399,7 +504,8 @@ __global__ void __maxnreg__(OZ_MAX_REGS) ozaki_syrk_kernel(OzArgs a) {
     extern __shared__ uint8_t oz_raw[];
     __shared__ OzShared S;
     uint8_t *smA = reinterpret_cast<uint8_t *>(((uintptr_t)oz_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t *smB = smA + (size_t)OZ_MAX_SLICES * OZ_A_BYTES;
+    uint8_t *smB = smA + (size_t)OZ_MAX_DIGITS * OZ_A_BYTES;
+    uint8_t *smC = smB + (size_t)OZ_STAGES * OZ_TILE_B;
     const int tid = threadIdx.x, warp = tid >> 5;
     const long t_begin = a.tiles * blockIdx.x / gridDim.x, t_end = a.tiles * (blockIdx.x + 1) / gridDim.x;
     if (t_begin >= t_end) return;
@@ -409,11 +515,14 @@ __global__ void __maxnreg__(OZ_MAX_REGS) ozaki_syrk_kernel(OzArgs a) {
         mbar_init(&S.fin, 1);
         for (int st = 0; st < OZ_STAGES; ++st) {
             mbar_init(&S.barB[st], 1);
-            mbar_init(&S.bfree[st], 1);
+            mbar_init(&S.done[st], 1);
         }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(&S.tfull[b], 1);
             mbar_init(&S.tempty[b], OZ_EPI_WARPS);
+        }
+        for (int st = 0; st < OZ_C_STAGES; ++st) {
+            mbar_init(&S.cfull[st], 1);
+            mbar_init(&S.cempty[st], OZ_EPI_WARPS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -427,14 +536,21 @@ __global__ void __maxnreg__(OZ_MAX_REGS) ozaki_syrk_kernel(OzArgs a) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    int I, J;
+    oz_tile_at(t_begin, a.nI, a.nJ, I, J);
+    const int ntile = (int)(t_end - t_begin);
     if (warp == 0) {
-        if ((tid & 31) == 0) oz_producer(a, S, smA, smB, t_begin, t_end);
+        if ((tid & 31) == 0) oz_mma(a, S, smA, smB, I, J, ntile);
         __syncwarp();
+    } else if (warp == OZ_AB_WARP) {
+        oz_load_ab(a, S, smA, smB, I, J, ntile);
+    } else if (warp == OZ_C_WARP) {
+        oz_load_c(a, S, smC, I, J, ntile);
     } else {
-        if (a.ns == OZ_MAX_SLICES)
-            oz_epilogue<OZ_MAX_SLICES>(a, S, t_begin, t_end);
+        if (a.nd == OZ_MAX_DIGITS)
+            oz_epilogue<OZ_MAX_DIGITS>(a, S, smC, I, J, ntile);
         else
-            oz_epilogue<0>(a, S, t_begin, t_end);
+            oz_epilogue<0>(a, S, smC, I, J, ntile);
     }
     tc_fence_before();
     __syncthreads();
@@ -444,11 +560,37 @@ __global__ void __maxnreg__(OZ_MAX_REGS) ozaki_syrk_kernel(OzArgs a) {
     }
 }
 
-// Digits of 32 rows per CTA; warp c takes K bytes 16c..16c+15.  Each
-// 16-byte group goes to both layouts: slice by slice (slices) and by
-// 16-row block, the block's ns slices back to back (slices_b).
-__global__ void __launch_bounds__(128) ozaki_split_kernel(const dd_t *P, long ldp, int n, int k, int ns, int8_t *slices, int8_t *slices_b, long slice_stride,
-                                                          int *exps) {
+// |x| 2^(120-e) truncated to an integer, with x's sign, for |x| 2^-e < 1/2:
+// the significand of x (53 bits) shifted.  A value that is not finite gives 0.
+__device__ __forceinline__ __int128 oz_fixed(double x, int e) {
+    const long long bits = __double_as_longlong(x);
+    const int ex = (int)((bits >> 52) & 0x7ff);
+    if (ex == 0x7ff) return 0;
+    const unsigned long long m = (unsigned long long)(bits & 0xfffffffffffffll) | (ex ? 1ull << 52 : 0ull);
+    const int q = max(ex, 1) - 1075 + 120 - e;
+    unsigned __int128 u = 0;
+    if (q >= 0) u = (unsigned __int128)m << min(q, 127);
+    else if (q > -64) u = m >> -q;
+    return bits < 0 ? -(__int128)u : (__int128)u;
+}
+
+// Byte k of four words, for k = 0..3: a 4 x 4 byte transpose.
+__device__ __forceinline__ void oz_transpose4(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t *o) {
+    const uint32_t ab0 = __byte_perm(a, b, 0x5140), ab1 = __byte_perm(a, b, 0x7362);
+    const uint32_t cd0 = __byte_perm(c, d, 0x5140), cd1 = __byte_perm(c, d, 0x7362);
+    o[0] = __byte_perm(ab0, cd0, 0x5410);
+    o[1] = __byte_perm(ab0, cd0, 0x7632);
+    o[2] = __byte_perm(ab1, cd1, 0x5410);
+    o[3] = __byte_perm(ab1, cd1, 0x7632);
+}
+
+// Digits of 32 rows per CTA; warp c takes K bytes 16c..16c+15.  An entry is
+// a 120-bit fixed-point integer U = P(r,k) 2^(120-e); with 128 added to the
+// bytes of digits 1 .. nd and to the next lower one (the rounding of the last
+// digit), the bytes are the digits plus 128.
+// A digit after the other peeled in dd arithmetic (10 FP64 operations each)
+// and written in two layouts took 14.6 us at n = 5003; this takes 6.8.
+__global__ void __launch_bounds__(128) ozaki_split_kernel(const dd_t *P, long ldp, int n, int k, int nd, int8_t *digits, int *exps) {
     __shared__ double rmax[4][32];
     const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
     const int r = blockIdx.x * 32 + lane;
@@ -466,27 +608,32 @@ __global__ void __launch_bounds__(128) ozaki_split_kernel(const dd_t *P, long ld
     int e = 0;
     if (m > 0.0) {
         int E;
-        frexp(m, &E); // m < 2^E, so |P| 2^-(E+1) <= 1/2
-        e = E + 1;
+        const double f = frexp(m, &E); // m = f 2^E, 1/2 <= f < 1
+        e = E + (f > 0.996 ? 2 : 1);   // |P| 2^-e <= 0.498
     }
     if (c == 0) exps[r] = e;
+    // byte p (0 .. 14) holds digit 15 - p: bytes 14 .. 15 - nd and one below
+    unsigned __int128 bias = 0;
+    for (int p = 14; p >= max(0, 14 - nd); --p) bias |= (unsigned __int128)0x80u << (8 * p);
+    uint32_t w[4][16]; // w[j][q]: word j of value q, its bytes the digits plus 128
 #pragma unroll
-    for (int q = 0; q < 16; ++q) x[q] = dd_make(ldexp(x[q].hi, 7 - e), ldexp(x[q].lo, 7 - e));
-    const int within = ((r >> 3) & 1) * 512 + c * 128 + (r & 7) * 16; // offset inside a 16-row block of one slice
-    int8_t *dst = slices + (long)(r >> 4) * 1024 + within;
-    int8_t *dstb = slices_b + (long)(r >> 4) * ns * 1024 + within;
-    for (int s = 0; s < ns; ++s) {
-        uint32_t w[4] = {0u, 0u, 0u, 0u};
+    for (int q = 0; q < 16; ++q) {
+        const unsigned __int128 u = (unsigned __int128)(oz_fixed(x[q].hi, e) + oz_fixed(x[q].lo, e)) + bias;
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const double d = rint(x[q].hi);
-            w[q >> 2] |= ((uint32_t)((int)d) & 0xffu) << (8 * (q & 3));
-            double err, sum = ddm::two_sum(x[q].hi - d, x[q].lo, err);
-            x[q] = dd_make(sum * 128.0, err * 128.0);
+        for (int j = 0; j < 4; ++j) w[j][q] = (uint32_t)(u >> (32 * j)) ^ 0x80808080u;
+    }
+    const int within = ((r >> 3) & 1) * 512 + c * 128 + (r & 7) * 16; // offset inside a 16-row block of one digit
+    int8_t *dst = digits + (long)(r >> 4) * nd * 1024 + within;
+#pragma unroll
+    for (int j = 3; j >= 0; --j) {
+        uint32_t o[4][4]; // o[g][b]: byte b of the word of values 4g .. 4g+3
+#pragma unroll
+        for (int g = 0; g < 4; ++g) oz_transpose4(w[j][4 * g], w[j][4 * g + 1], w[j][4 * g + 2], w[j][4 * g + 3], o[g]);
+#pragma unroll
+        for (int b = 3; b >= 0; --b) {
+            const int s = 15 - (4 * j + b); // digit
+            if (s >= 1 && s <= nd) *reinterpret_cast<uint4 *>(dst + (long)(s - 1) * 1024) = make_uint4(o[0][b], o[1][b], o[2][b], o[3][b]);
         }
-        const uint4 v = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4 *>(dst + (long)s * slice_stride) = v;
-        *reinterpret_cast<uint4 *>(dstb + (long)s * 1024) = v;
     }
 }
 
@@ -497,19 +644,17 @@ void ozaki_syrk_sub_lower(cudaStream_t st, const dd_t *P, long ldp, int n, int k
     if (k > OZ_K) throw Error(ERR_ARG, "ozaki: panel wider than 64 columns");
     if (w.slices_used < 8 || w.slices_used > OZ_MAX_SLICES) throw Error(ERR_ARG, "ozaki: slice count must be 8..16");
     const int rows = (int)(ceil_div(n, OZ_ROWS_A) * OZ_ROWS_A);
-    if (rows > w.row_cap || !w.slices || !w.slices_b || !w.exps || !w.err) throw Error(ERR_ARG, "ozaki: workspace smaller than the panel");
-    const long stride = (long)w.row_cap * OZ_K;
-    ozaki_split_kernel<<<rows / 32, 128, 0, st>>>(P, ldp, n, k, w.slices_used, w.slices, w.slices_b, stride, w.exps);
+    if (rows > w.row_cap || !w.digits || !w.exps || !w.err) throw Error(ERR_ARG, "ozaki: workspace smaller than the panel");
+    const int nd = ozaki_digits(w.slices_used);
+    ozaki_split_kernel<<<rows / 32, 128, 0, st>>>(P, ldp, n, k, nd, w.digits, w.exps);
     CK_LAUNCH();
     OzArgs a;
-    a.slices = w.slices;
-    a.slices_b = w.slices_b;
-    a.slice_stride = stride;
+    a.digits = w.digits;
     a.exps = w.exps;
     a.C = C;
     a.ldc = ldc;
     a.n = n;
-    a.ns = w.slices_used;
+    a.nd = nd;
     a.nI = rows / OZ_ROWS_A;
     a.nJ = (int)ceil_div(n, OZ_COLS_B);
     a.skip = skip;

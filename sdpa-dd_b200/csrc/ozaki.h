@@ -1,5 +1,5 @@
 // Tensor-core split of the Cholesky trailing update: C(lower) -= P P^T with
-// dd operands cut into signed 7-bit integer slices (an Ozaki-style
+// dd operands cut into signed integer digits (an Ozaki-style
 // error-free split) and multiplied on the INT8 tensor cores (tcgen05,
 // kind::i8) with exact int32 accumulation, then rebuilt in dd.
 #pragma once
@@ -7,16 +7,18 @@
 
 namespace sddd {
 
-constexpr int OZ_MAX_SLICES = 16;
+constexpr int OZ_MAX_SLICES = 16; // 7-bit slices a caller may ask for
+// base-256 digits that carry `slices` 7-bit slices in the trailing update
+constexpr int ozaki_digits(int slices) { return (7 * slices + 7) / 8; }
+constexpr int OZ_MAX_DIGITS = ozaki_digits(OZ_MAX_SLICES);
 constexpr int OZ_K = 64;        // panel width the split handles (K of the update)
 constexpr int OZ_ROWS_A = 128;  // output tile rows (MMA M)
-constexpr int OZ_COLS_B = 16;   // output tile columns (per B slice)
+constexpr int OZ_COLS_B = 16;   // output tile columns (per B digit)
 
-// Device workspace of the split: slices for `row_cap` rows (a multiple of
+// Device workspace of the split: digits for `row_cap` rows (a multiple of
 // 128), row exponents and an error word.
 struct OzakiWork {
-    int8_t *slices = nullptr; // OZ_MAX_SLICES x row_cap x 64 bytes, tiled, slice by slice
-    int8_t *slices_b = nullptr; // the same digits by 16-row block: each block's slices contiguous
+    int8_t *digits = nullptr; // row_cap x OZ_MAX_DIGITS x 64 bytes by 16-row block: each block's digits contiguous
     int *exps = nullptr;      // row_cap
     int *err = nullptr;       // 0, or the code of a wait that gave up
     int *h_err = nullptr;     // pinned host word for reading err (or null)
