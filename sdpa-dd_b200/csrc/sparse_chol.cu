@@ -15,12 +15,11 @@
 // entry thus sees its updates in ascending pivot order, one dd multiply and
 // one dd subtract each, and is scaled once, when its column becomes the
 // pivot.  Here, per panel J of 64 pivots:
-//   sp_panel_kernel   one CTA per tile of column block J (the diagonal
-//                     tile first): every CTA factors the diagonal tile in
-//                     shared memory (pivots in order, the next column's
-//                     pivot chain beside the other columns' updates), and
-//                     CTA k > 0 carries its own tile below with the same
-//                     pivots;
+//   sp_panel_kernel   one CTA for the diagonal tile of column block J and two
+//                     per tile below: every CTA factors the diagonal tile
+//                     (pivots in order, the next column's pivot chain beside
+//                     the other columns' updates), and the others carry half
+//                     a tile below with the same pivots;
 //   sp_update_kernel  every tile (I, K), K > J, that some column of J
 //                     reaches in both I and K: entry (a, r) -= L(r,b) L(a,b)
 //                     for the columns b of J ascending, where both are in
@@ -41,6 +40,7 @@
 
 #include <algorithm>
 
+#include "fastdiv.cuh"
 #include "prof.h"
 
 namespace sddd {
@@ -108,75 +108,112 @@ __global__ void sp_gather_kernel(const dd_t *tiles, const int *ent_b, const int 
 }
 
 // ------------------------------------------------------------ panel
-// CTA 0: the diagonal tile of panel J; CTA k > 0: the diagonal tile again
-// (identical arithmetic) and below-diagonal tile col_tiles[k - 1].  Every
-// CTA reads the unfactored diagonal tile at its start, so the factored one
-// is written back by the CTA that finishes last (counted in done[J], which
-// it resets for the next factorisation).
-// Step k (one barrier): warp 0 takes column k+1 through pivot k's update,
-// its own pivot (1/sqrt) and its scaling, while warps 1.. apply pivot k's
-// update to columns k+2.. (one column per warp at a time, rows over the
-// lanes); so the chain of pivots runs beside the bulk of the updates and
-// every entry still sees pivot k's update before pivot k+1's.
+// CTA 0: the diagonal tile of panel J; CTA 1 + 2 k + h: the diagonal tile
+// again (identical arithmetic) and rows 32 h .. 32 h + 31 of below-diagonal
+// tile col_tiles[k].  Every CTA reads the unfactored diagonal tile at its
+// start, so the factored one is written back by the CTA that finishes last
+// (counted in done[J], which it resets for the next factorisation).
+// Step c (one barrier): warp 0 publishes column c, the other warps apply its
+// update to columns c+2.. (a column a warp at a time, rows over the lanes)
+// while warp 0 takes column c+1 through it in registers and forms, in all its
+// lanes, the next diagonal entry and its 1/sqrt; so the chain of pivots (a
+// square root and reciprocal, a scaling, a product and a subtraction a column)
+// runs beside the bulk of the updates, alone on its SM sub-partition (warps 4,
+// 8, .. have no work), and every entry still sees pivot k's update before
+// pivot k+1's.
+// Chain of 200 blocks of order 20: 46 us a panel; with a whole tile below
+// a CTA, the column through shared memory between its steps and the plain
+// root and quotient on lane 0 75.
 constexpr int SP_PANEL_THREADS = 512;
+constexpr int SPH = SP_T / 2, SPHL = SPH + 1; // rows of a half tile, its leading dimension
+constexpr size_t SP_PANEL_SMEM = SP_TILE_SMEM + sizeof(double2) * SPHL * SP_T;
 __global__ void __launch_bounds__(SP_PANEL_THREADS) sp_panel_kernel(dd_t *tiles, const unsigned long long *mask, int m, int J, int diag_t,
                                                                     const int *col_tiles, int *done) {
     extern __shared__ double2 sp_sm[];
     double2 *D = sp_sm;
-    double2 *U = sp_sm + SP_T * SPL; // used only when the CTA has a tile below (ut >= 0, mu != 0)
-    __shared__ unsigned long long md[SP_T], mu[SP_T];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    double2 *U = sp_sm + SP_T * SPL; // used only when the CTA has rows below (ut >= 0, mu != 0)
+    __shared__ unsigned long long md[SP_T];
+    __shared__ uint32_t mu[SP_T];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nb = min(SP_T, m - J * SP_T);
-    const int ut = blockIdx.x > 0 ? col_tiles[blockIdx.x - 1] : -1;
+    const int ut = blockIdx.x > 0 ? col_tiles[(blockIdx.x - 1) / 2] : -1;
+    const int u0 = (blockIdx.x - 1) % 2 * SPH;
+    dd_t *Ug = tiles + (long)max(ut, 0) * SP_T * SP_T + max(u0, 0);
+    if (ut >= 0)
+        for (int e = tid; e < SPH * SP_T; e += SP_PANEL_THREADS) {
+            const int i = e % SPH, j = e / SPH;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(U + i + SPHL * j)), "l"(Ug + i + SP_T * j) : "memory");
+        }
     sp_load_tile(D, tiles + (long)diag_t * SP_T * SP_T, tid, blockDim.x);
-    if (ut >= 0) sp_load_tile(U, tiles + (long)ut * SP_T * SP_T, tid, blockDim.x);
     if (tid < SP_T) {
         md[tid] = mask[(long)diag_t * SP_T + tid];
-        mu[tid] = ut >= 0 ? mask[(long)ut * SP_T + tid] : 0ull;
+        mu[tid] = ut >= 0 ? (uint32_t)(mask[(long)ut * SP_T + tid] >> u0) : 0u;
     }
     __syncthreads();
-    // warp 0: column c's pivot d_c = 1/sqrt(B(c,c)) (0 for a negative
-    // pivot) and the scaling of column c by it
-    auto pivot = [&](int c) {
-        double ih = 0.0, il = 0.0;
-        if (lane == 0) {
-            const dd_t d = sm_dd(D, c, c);
-            const dd_t inv = dd_lt_d(d, 0.0) ? dd_zero() : dd_div(dd_from(1.0), dd_sqrt(d));
-            sm_st(D, c, c, inv);
-            ih = inv.hi;
-            il = inv.lo;
-        }
-        const dd_t inv = dd_make(__shfl_sync(0xffffffffu, ih, 0), __shfl_sync(0xffffffffu, il, 0));
-        const unsigned long long cc = md[c], uc = mu[c];
-        for (int i = lane; i < SP_T; i += 32) {
-            if (i > c && bit64(cc, i)) sm_st(D, i, c, dd_muleq(sm_dd(D, i, c), inv));
-            if (bit64(uc, i)) sm_st(U, i, c, dd_muleq(sm_dd(U, i, c), inv));
-        }
-        __syncwarp();
+    auto u_dd = [&](int j) {
+        const double2 v = U[lane + SPHL * j];
+        return dd_make(v.x, v.y);
     };
-    // pivot k's update of column r (r in struct(k)): entry (i, r) -= L(r,k) L(i,k)
-    auto apply = [&](int k, int r, unsigned long long ck, unsigned long long uk) {
-        const dd_t lrk = sm_dd(D, r, k);
-        for (int i = lane; i < SP_T; i += 32) {
-            if (i >= r && bit64(ck, i)) sm_st(D, i, r, dd_sub(sm_dd(D, i, r), dd_mul(lrk, sm_dd(D, i, k))));
-            if (bit64(uk, i)) sm_st(U, i, r, dd_sub(sm_dd(U, i, r), dd_mul(lrk, sm_dd(U, i, k))));
+    auto u_st = [&](int j, dd_t v) { U[lane + SPHL * j] = make_double2(v.hi, v.lo); };
+    const int ia = lane, ib = lane + 32; // this lane's rows of D
+    if (warp == 0) {
+        // column c through the pivots before it, and its diagonal entry in every lane
+        dd_t xa = sm_dd(D, ia, 0), xb = sm_dd(D, ib, 0), xu = mu[0] ? u_dd(0) : dd_zero(), d = sm_dd(D, 0, 0);
+        for (int c = 0; c < nb; ++c) {
+            dd_t l, inv; // d_c = 1/sqrt(B(c,c)), 0 for a negative pivot
+            if (!sqrt_rcp_fast(d, l, inv)) {
+                if (dd_lt_d(d, 0.0)) inv = dd_zero();
+                else sqrt_rcp_plain(d, l, inv);
+            }
+            const unsigned long long cc = md[c];
+            const uint32_t uc = mu[c];
+            const dd_t la = dd_muleq(xa, inv), lb = dd_muleq(xb, inv), lu = dd_muleq(xu, inv);
+            const int cn = min(c + 1, SP_T - 1);
+            const bool next = bit64(cc, cn);
+            const dd_t ln = dd_make(__shfl_sync(0xffffffffu, cn < 32 ? la.hi : lb.hi, cn & 31), __shfl_sync(0xffffffffu, cn < 32 ? la.lo : lb.lo, cn & 31));
+            if (ia > c && bit64(cc, ia)) sm_st(D, ia, c, la);
+            if (ib > c && bit64(cc, ib)) sm_st(D, ib, c, lb);
+            if (lane == 0) sm_st(D, c, c, inv);
+            if (bit64(uc, lane)) u_st(c, lu);
+            __syncthreads(); // column c is published, column c+1 has seen pivot c-1
+            if (c + 1 >= nb) break;
+            d = sm_dd(D, cn, cn);
+            xa = sm_dd(D, ia, cn);
+            xb = sm_dd(D, ib, cn);
+            if (mu[cn]) xu = u_dd(cn);
+            if (next) {
+                d = dd_sub(d, dd_mul(ln, ln));
+                const dd_t ya = dd_sub(xa, dd_mul(ln, la)), yb = dd_sub(xb, dd_mul(ln, lb)), yu = dd_sub(xu, dd_mul(ln, lu));
+                if (ia >= cn && bit64(cc, ia)) xa = ya;
+                if (ib >= cn && bit64(cc, ib)) xb = yb;
+                if (bit64(uc, lane)) xu = yu;
+            }
         }
-    };
-    if (warp == 0 && nb > 0) pivot(0);
-    __syncthreads();
-    for (int k = 0; k + 1 < nb; ++k) {
-        const unsigned long long ck = md[k], uk = mu[k];
-        if (warp == 0) {
-            if (bit64(ck, k + 1)) apply(k, k + 1, ck, uk);
-            __syncwarp();
-            pivot(k + 1);
-        } else {
-            for (int r = k + 1 + warp; r < nb; r += nw - 1)
-                if (bit64(ck, r)) apply(k, r, ck, uk);
+    } else {
+        const int h = (warp >> 2) * 3 + (warp & 3) - 1, nh = SP_PANEL_THREADS / 32 / 4 * 3;
+        for (int c = 0; c < nb; ++c) {
+            __syncthreads();
+            if ((warp & 3) == 0) continue;
+            const unsigned long long cc = md[c];
+            const uint32_t uc = mu[c];
+            const bool ba = bit64(cc, ia), bb = bit64(cc, ib), bu = bit64(uc, lane);
+            const dd_t la = sm_dd(D, ia, c), lb = sm_dd(D, ib, c), lu = uc ? u_dd(c) : dd_zero();
+            for (int r = c + 2 + h; r < nb; r += nh) {
+                if (!bit64(cc, r)) continue;
+                // entry (i, r) -= L(r,c) L(i,c)
+                const dd_t lr = sm_dd(D, r, c);
+                if (ba && ia >= r) sm_st(D, ia, r, dd_sub(sm_dd(D, ia, r), dd_mul(lr, la)));
+                if (bb && ib >= r) sm_st(D, ib, r, dd_sub(sm_dd(D, ib, r), dd_mul(lr, lb)));
+                if (bu) u_st(r, dd_sub(u_dd(r), dd_mul(lr, lu)));
+            }
         }
-        __syncthreads();
     }
-    if (ut >= 0) sp_store_tile(tiles + (long)ut * SP_T * SP_T, U, tid, blockDim.x);
+    __syncthreads();
+    if (ut >= 0)
+        for (int e = tid; e < SPH * SP_T; e += SP_PANEL_THREADS) {
+            const int i = e % SPH, j = e / SPH;
+            *reinterpret_cast<double2 *>(Ug + i + SP_T * j) = U[i + SPHL * j];
+        }
     __shared__ int last;
     if (tid == 0) last = atomicAdd(done + J, 1) == (int)gridDim.x - 1;
     __syncthreads();
@@ -503,7 +540,7 @@ void sparse_setup_structure(Context &c, const SparseStructure &ss) {
 static void sparse_launches(Context &c, cudaGraph_t g) {
     SparseDev &s = *c.sp;
     const TileSchedule &t = s.sched;
-    CK(cudaFuncSetAttribute(sp_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SP_TWO_TILES));
+    CK(cudaFuncSetAttribute(sp_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SP_PANEL_SMEM));
     CK(cudaFuncSetAttribute(sp_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SP_TWO_TILES));
     std::vector<cudaGraphNode_t> last_writer(t.ntiles, nullptr);
     std::vector<std::vector<cudaGraphNode_t>> into(t.nblk);
@@ -519,7 +556,7 @@ static void sparse_launches(Context &c, cudaGraph_t g) {
     for (int J = 0; J < t.nblk; ++J) {
         const int ncol = t.col_ptr[J + 1] - t.col_ptr[J];
         int diag = t.tile_of[J + (size_t)t.nblk * J];
-        const size_t smem = ncol > 0 ? SP_TWO_TILES : SP_TILE_SMEM;
+        const size_t smem = ncol > 0 ? SP_PANEL_SMEM : SP_TILE_SMEM;
         const int *col = s.col_tiles.p + t.col_ptr[J];
         int Jv = J;
         cudaGraphNode_t pnode = nullptr;
@@ -527,7 +564,7 @@ static void sparse_launches(Context &c, cudaGraph_t g) {
             void *args[] = {&tiles, &mask, &m, &Jv, &diag, &col, &done};
             cudaKernelNodeParams kp{};
             kp.func = (void *)sp_panel_kernel;
-            kp.gridDim = dim3(1 + ncol);
+            kp.gridDim = dim3(1 + 2 * ncol);
             kp.blockDim = dim3(SP_PANEL_THREADS);
             kp.sharedMemBytes = (unsigned)smem;
             kp.kernelParams = args;
