@@ -40,7 +40,8 @@ void zero_upper(cudaStream_t st, dd_t *A, long lda, int n, int batch = 1, long s
 // *info_dev to a failing column.
 void potrf_batched(cudaStream_t st, dd_t *A, long lda, int n, long sA, int batch, int *info_dev);
 // Progress words of the one-launch triangular solve: one flag per 64-entry
-// block (the epoch of the solve that finished it), then an error word.
+// block (the epoch of the solve that finished it), then an error word; and
+// the blocked solves' published entries, with the epoch beside them.
 // The owner zeroes them once; the epoch advances with every solve.
 struct TrsvSync {
     int *flags = nullptr; // capacity flags + 1 error word
@@ -49,8 +50,10 @@ struct TrsvSync {
     int *h_err = nullptr; // pinned host word for reading the error word (or null)
     cudaEvent_t wait_ev = nullptr; // blocking-sync event to wait on (or null: stream sync)
     unsigned long long wait_ns = 2000000000ull; // budget of one wait for a block
-    int withhold = -1; // tests of the bounded waits: this block's flag is never published
+    int withhold = -1; // tests of the bounded waits: this block is never published
+    unsigned long long *xch = nullptr; // TRSV_XCH_BLOCK words per 64-entry block
 };
+constexpr size_t TRSV_XCH_BLOCK = 64 * 4;
 // x = L^-1 x ('N') or L^-T x ('T'), L lower, as Rtrsv("Lower", trans, "NonUnit").
 // shared_gpu: other streams keep the GPU busy (a batch worker); short
 // solves then run in one CTA with an ordinary launch.
@@ -67,8 +70,9 @@ void trsv_check(cudaStream_t st, const TrsvSync &sync);
 void trsv_diag_inverse(cudaStream_t st, const dd_t *L, long lda, int n, dd_t *W);
 // x = L^-1 x ('N') or L^-T x ('T') by blocks, with W from
 // trsv_diag_inverse: one cooperative launch; the same progress words and
-// error reporting (trsv_check) as trsv_lower.  Not Rtrsv's operation order.
-void trsv_blocked(cudaStream_t st, char trans, const dd_t *L, long lda, int n, const dd_t *W, dd_t *x, TrsvSync &sync);
+// error reporting (trsv_check) as trsv_lower, and the same right-hand sides
+// side by side.  Not Rtrsv's operation order.
+void trsv_blocked(cudaStream_t st, char trans, const dd_t *L, long lda, int n, const dd_t *W, dd_t *x, TrsvSync &sync, int nrhs = 1, long ldx = 0);
 void inv_lower(cudaStream_t st, const dd_t *L, long lda, int n, dd_t *X, long ldx, int batch = 1, long sL = 0, long sX = 0);
 void trmm_lt(cudaStream_t st, const dd_t *M, long ldm, int n, dd_t *B, long ldb, int batch = 1, long sM = 0, long sB = 0);
 void symmetrize(cudaStream_t st, dd_t *A, int n, int batch = 1, long sA = 0);

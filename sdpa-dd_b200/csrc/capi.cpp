@@ -774,8 +774,9 @@ int sddd_Rpotrs(sddd_ctx *ctx, char uplo, long n, long nrhs, const sddd_dd *A, l
         if (n == 0 || nrhs == 0) return SDDD_OK;
         sddd::Context &c = *ctx->c;
         const dd_t *L = reinterpret_cast<const dd_t *>(A);
-        // plain form: groups of right-hand sides side by side, a few CTAs each
-        const int group = c.tc_slices > 0 ? 1 : (int)std::min(nrhs, 8L);
+        // groups of right-hand sides side by side, a few CTAs each (in the
+        // split form a CTA fills an SM)
+        const int group = (int)std::min(nrhs, c.tc_slices > 0 ? 4L : 8L);
         sddd::TrsvSync &sync = sddd::trsv_sync(c, (int)n, group);
         if (c.tc_slices > 0) {
             // the split form's blocked solves; the inverted diagonal blocks
@@ -784,10 +785,11 @@ int sddd_Rpotrs(sddd_ctx *ctx, char uplo, long n, long nrhs, const sddd_dd *A, l
             c.winv_valid = false;
             c.trsv_winv.alloc((size_t)sddd::ceil_div(n, 64L) * 64 * 64);
             sddd::trsv_diag_inverse(c.stream, L, lda, (int)n, c.trsv_winv.p);
-            for (long r = 0; r < nrhs; ++r) {
+            for (long r = 0; r < nrhs; r += group) {
                 dd_t *x = reinterpret_cast<dd_t *>(B) + ldb * r;
-                sddd::trsv_blocked(c.stream, 'N', L, lda, (int)n, c.trsv_winv.p, x, sync);
-                sddd::trsv_blocked(c.stream, 'T', L, lda, (int)n, c.trsv_winv.p, x, sync);
+                const int g = (int)std::min<long>(group, nrhs - r);
+                sddd::trsv_blocked(c.stream, 'N', L, lda, (int)n, c.trsv_winv.p, x, sync, g, ldb);
+                sddd::trsv_blocked(c.stream, 'T', L, lda, (int)n, c.trsv_winv.p, x, sync, g, ldb);
             }
         } else {
             for (long r = 0; r < nrhs; r += group) {

@@ -154,9 +154,11 @@ TrsvSync &trsv_sync(Context &c, int n, int nrhs) {
     const int nblk = (int)ceil_div(n, 64) * nrhs;
     if (nblk > c.trsv.capacity || !c.trsv.flags) {
         CK(cudaStreamSynchronize(c.stream));
-        c.trsv_flags.alloc((size_t)nblk + 1);
-        CK(cudaMemsetAsync(c.trsv_flags.p, 0, sizeof(int) * ((size_t)nblk + 1), c.stream));
+        const size_t words = ((size_t)nblk + 1 + 3) / 4 * 4, xch = (size_t)nblk * TRSV_XCH_BLOCK;
+        c.trsv_flags.alloc(words + 2 * xch);
+        CK(cudaMemsetAsync(c.trsv_flags.p, 0, sizeof(int) * (words + 2 * xch), c.stream));
         c.trsv = TrsvSync{c.trsv_flags.p, nblk, 0, static_cast<int *>(c.h_pin), c.sync_ev};
+        c.trsv.xch = reinterpret_cast<unsigned long long *>(c.trsv_flags.p + words);
     }
     c.trsv.wait_ns = c.wait_ns;
     c.trsv.withhold = c.withhold_block;

@@ -16,12 +16,21 @@
 // solve order).  For each of its blocks it streams the tiles L(c,p) (or
 // L(p,c)) and finally W_c into shared memory with bulk copies (one copy per
 // tile column of up to 1 KB, three tiles in flight, completion on an
-// mbarrier), waits for block p's flag (release/acquire, bounded), and all
-// 256 threads multiply: thread (r, q) sums the 16 products of row r (or
-// column r) in quarter q of the tile into its own running dd sum, so a tile
-// costs a 16-step chain and the critical path per block is one tile and
-// three 64 x 64 products (W_c, L(c,c), W_c), each a 16-step chain and a
-// 4-way combination.  L is read once per solve.
+// mbarrier), waits (bounded) for block p's entries, which carry the solve's epoch, and
+// all 256 threads multiply: thread (r, q) sums every fourth product of row r
+// (or column r), so the critical path per block is one tile and three triangular
+// 64 x 64 products (W_c, L(c,c), W_c), each followed by a 4-way combination.
+// L is read once per solve.  Right-hand sides go side by side (grid row y).
+//
+// What bounds a block is one SM's FP64 issue rate: 4096 products and sums in
+// dd operations are 29 instructions each, 1.9k cycles.  So a thread's sum is
+// a compensated one (Ogita, Rump, Oishi, "Accurate sum and dot product",
+// SIAM J. Sci. Comput. 26, 2005): the high parts' products summed with their
+// rounding errors collected beside (12 instructions a term, and a chain of
+// one addition), rounded to a dd per thread.
+// Measured, n = 5003: 426 us for one solve or two side by side; with dd sums of 16
+// consecutive terms, all of W_c multiplied, the quarters' sums through shared memory
+// and a flag per block 583; n = 9980 840, before 1144.
 //
 // Every wait is bounded (the solve's wait budget, 2 s by default); a CTA
 // that gives up records the awaited block in the error word (read by
@@ -38,7 +47,8 @@ namespace {
 constexpr int TB = 64;           // block order
 constexpr int TB_LD = 65;        // padded leading dimension of a tile in shared memory
 constexpr int TB_STAGES = 3;     // tiles in flight per CTA
-constexpr int TB_THREADS = 256;  // (row, quarter) pairs of a tile
+constexpr int TB_Q = 4;          // threads that share a row of a tile
+constexpr int TB_THREADS = TB * TB_Q;
 constexpr int TB_TILE = TB * TB_LD; // double2 per stage
 
 struct TbShared {
@@ -46,7 +56,7 @@ struct TbShared {
     int fail;
     long fail_at; // the first tile not consumed when the CTA gave up
 };
-constexpr size_t TB_SMEM = sizeof(double2) * ((size_t)TB_STAGES * TB_TILE + 3 * TB + 4 * TB) + 128;
+constexpr size_t TB_SMEM = sizeof(double2) * ((size_t)TB_STAGES * TB_TILE + 3 * TB) + 128;
 static_assert(TB_SMEM <= 232448, "blocked solve: shared memory above the per-CTA limit");
 
 struct TbArgs {
@@ -55,9 +65,11 @@ struct TbArgs {
     const dd_t *W; // nblk tiles of TB x TB (leading dimension TB): L(c,c)^-1, lower
     int n, nblk, epoch, trans; // trans: 0 'N', 1 'T'
     dd_t *x;
-    int *flags, *err;
+    unsigned long long *xch; // published entries: TB_REC words each
+    int *err;
     unsigned long long wait_ns;
-    int withhold; // a block whose flag is never published (-1: none)
+    int withhold; // a block that is never published (-1: none)
+    long ldx;     // between right-hand sides
 };
 
 // The k-th tile block c reads: 'N' L(c, k) for k < c, 'T' L(nblk-1-k, c)
@@ -119,12 +131,37 @@ __device__ __forceinline__ int tb_ld_acquire(const int *p) {
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void tb_st_release(int *p, int v) { asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
 
-// Bounded wait for block p's flag (thread 0 only).
-__device__ bool tb_wait_flag(const TbArgs &a, int p) {
+// A published entry: its four 32-bit words, each in the upper half of a 64-bit
+// word whose lower half is the solve's epoch.  64-bit accesses are single, so a
+// reader that finds the epoch in all four has the entry, without a fence and a
+// second round trip behind a flag.
+constexpr int TB_REC = 4;
+static_assert((size_t)TB * TB_REC == TRSV_XCH_BLOCK, "published words of a block");
+__device__ __forceinline__ void tb_publish(unsigned long long *rec, int epoch, dd_t v) {
+    const unsigned long long e = (unsigned)epoch, h = (unsigned long long)__double_as_longlong(v.hi), l = (unsigned long long)__double_as_longlong(v.lo);
+    const unsigned long long up = 0xffffffff00000000ull;
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(rec), "l"((h & up) | e), "l"((h << 32) | e) : "memory");
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(rec + 2), "l"((l & up) | e), "l"((l << 32) | e) : "memory");
+}
+__device__ __forceinline__ bool tb_read(const unsigned long long *rec, int epoch, double2 &v) {
+    unsigned long long a, b, c, d;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(rec) : "memory");
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(c), "=l"(d) : "l"(rec + 2) : "memory");
+    const unsigned e = (unsigned)epoch;
+    const unsigned long long up = 0xffffffff00000000ull;
+    v.x = __longlong_as_double((long long)((a & up) | (b >> 32)));
+    v.y = __longlong_as_double((long long)((c & up) | (d >> 32)));
+    return (unsigned)a == e && (unsigned)b == e && (unsigned)c == e && (unsigned)d == e;
+}
+
+// Bounded wait for an entry.  The error word and the clock are looked at once
+// in a while only: either costs as much as a look at the entry.
+__device__ bool tb_wait_entry(const TbArgs &a, const unsigned long long *rec, double2 &v) {
+    for (int k = 0; k < 64; ++k)
+        if (tb_read(rec, a.epoch, v)) return true;
     const unsigned long long t0 = globaltimer_ns();
-    while (tb_ld_acquire(a.flags + p) != a.epoch) {
+    while (!tb_read(rec, a.epoch, v)) {
         if (tb_ld_acquire(a.err) != 0 || globaltimer_ns() - t0 > a.wait_ns) return false;
         __nanosleep(20);
     }
@@ -138,38 +175,91 @@ __device__ __forceinline__ dd_t sm_dd(const double2 *T, int i) {
 
 __device__ __forceinline__ double2 tb_pack(dd_t v) { return make_double2(v.hi, v.lo); }
 
-// The four quarters' partial sums of entry i: (p0 + p1) + (p2 + p3).
-__device__ __forceinline__ dd_t tb_sum4(const double2 *part, int i) {
-    return dd_add(dd_add(sm_dd(part, i), sm_dd(part, TB + i)), dd_add(sm_dd(part, 2 * TB + i), sm_dd(part, 3 * TB + i)));
-}
-
-// Thread (r, q)'s part of row r of M y ('N') or of column r of M^T y ('T')
-// over the terms t2 of quarter q (t2 < nb); with lower, only M(i,j), i >= j.
-__device__ __forceinline__ double2 tb_matvec(const double2 *M, const double2 *y, int r, int q, int nb, int trans, bool lower) {
-    dd_t w = dd_zero();
-    if (r < nb) {
-        int lo = q * 16, hi = min(lo + 16, nb);
-        if (trans == 0) {
-            if (lower) hi = min(hi, r + 1);
-            for (int t2 = lo; t2 < hi; ++t2) w = dd_add(w, dd_mul(sm_dd(M, r + t2 * TB_LD), sm_dd(y, t2)));
-        } else {
-            if (lower) lo = max(lo, r);
-            for (int t2 = lo; t2 < hi; ++t2) w = dd_add(w, dd_mul(sm_dd(M, t2 + r * TB_LD), sm_dd(y, t2)));
+// A compensated sum of dd products: s + e + f, e the sum of the rounding errors
+// of s, f that of the products' low parts; folded every eight terms, so that
+// e and f stay an ulp or two of s (folded every tile only, the solve's error on
+// a factor of condition 1e8 was 12 % above that of dd sums).
+struct TbSum {
+    double s = 0.0, e = 0.0, f = 0.0;
+    __device__ __forceinline__ void add(double2 x, double2 y) {
+        const double p = __dmul_rn(x.x, y.x);
+        const double pe = __fma_rn(x.y, y.x, __fma_rn(x.x, y.y, __fma_rn(x.x, y.x, -p)));
+        double t;
+        s = ddm::two_sum(s, p, t);
+        e = __dadd_rn(e, t);
+        f = __dadd_rn(f, pe);
+    }
+    // s the rounded sum, e the rest
+    __device__ __forceinline__ void fold() {
+        double t;
+        e = ddm::two_sum(e, f, f);
+        s = ddm::two_sum(s, e, t);
+        e = __dadd_rn(t, f);
+        f = 0.0;
+    }
+    // the sum over a row's lanes
+    __device__ __forceinline__ void join() {
+#pragma unroll
+        for (int m = 32 / TB_Q; m < 32; m *= 2) {
+            double t, u;
+            s = ddm::two_sum(s, __shfl_xor_sync(0xffffffffu, s, m), t);
+            e = ddm::two_sum(e, __shfl_xor_sync(0xffffffffu, e, m), u);
+            f = __dadd_rn(__dadd_rn(f, __shfl_xor_sync(0xffffffffu, f, m)), u);
+            e = ddm::two_sum(e, t, u);
+            f = __dadd_rn(f, u);
         }
     }
-    return tb_pack(w);
+    __device__ __forceinline__ dd_t dd() const {
+        TbSum w = *this;
+        w.fold();
+        double l;
+        const double h = ddm::fast_two_sum(w.s, w.e, l);
+        return dd_make(h, l);
+    }
+};
+
+// Thread (r, q)'s part of row r of M y ('N') or of column r of M^T y ('T'):
+// the terms t2 = q, q + TB_Q, .. of [lo, hi).
+__device__ __forceinline__ void tb_dot(TbSum &w, const double2 *M, const double2 *y, int r, int q, int lo, int hi, int trans) {
+    int t2 = q + (max(lo - q, 0) + TB_Q - 1) / TB_Q * TB_Q;
+    const double2 *m = trans == 0 ? M + r : M + r * TB_LD;
+    const int ld = trans == 0 ? TB_LD : 1;
+#pragma unroll
+    for (int half = 1; half <= 2; ++half) {
+        const int end = min(hi, half * TB / 2);
+#pragma unroll 4
+        for (; t2 < end; t2 += TB_Q) w.add(m[t2 * ld], y[t2]);
+        w.fold();
+    }
+}
+
+// A row (or column) of a tile and the residue of its other index: a row's TB_Q
+// lanes lie in one warp, and eight neighbouring lanes read eight neighbouring
+// rows (columns), so different banks.
+__device__ __forceinline__ int tb_row(int warp, int lane) { return 8 * warp + (lane & 7); }
+__device__ __forceinline__ int tb_residue(int lane) { return lane >> 3; }
+static_assert(TB_Q == 4, "eight rows a warp");
+
+// Entry r of M y ('N') or M^T y ('T') for a lower triangular M (M(i,j), i >= j)
+// of order nb, in the row's lanes.
+__device__ __forceinline__ dd_t tb_lower(const double2 *M, const double2 *y, int r, int q, int nb, int trans) {
+    TbSum w;
+    if (r < nb) tb_dot(w, M, y, r, q, trans ? r : 0, trans ? nb : r + 1, trans);
+    w.join();
+    return w.dd();
 }
 
 __global__ void __launch_bounds__(TB_THREADS, 1) trsv_blocked_kernel(TbArgs a) {
     extern __shared__ __align__(128) double2 tb_sm[];
     double2 *tiles = tb_sm;                      // TB_STAGES x TB_TILE
-    double2 *xs = tiles + TB_STAGES * TB_TILE;   // TB: x of block p, then the residual v of block c
+    double2 *xs = tiles + TB_STAGES * TB_TILE;   // TB: x of block p, then v of block c
     double2 *x0 = xs + TB;                       // TB: W_c v
     double2 *rs = x0 + TB;                       // TB: v - L(c,c) x0
-    double2 *part = rs + TB;                     // 4 x TB partial sums
-    TbShared &S = *reinterpret_cast<TbShared *>(part + 4 * TB);
+    TbShared &S = *reinterpret_cast<TbShared *>(rs + TB);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int r = tid & (TB - 1), q = tid >> 6; // row (or column) of the tile, quarter of its other index
+    const int r = tb_row(warp, lane), q = tb_residue(lane);
+    a.x += a.ldx * blockIdx.y;
+    a.xch += (long)a.nblk * TB * TB_REC * blockIdx.y;
     if (tid == 0) {
         for (int s = 0; s < TB_STAGES; ++s) mbar_init(&S.bar[s], 1);
         S.fail = 0;
@@ -188,19 +278,24 @@ __global__ void __launch_bounds__(TB_THREADS, 1) trsv_blocked_kernel(TbArgs a) {
                 tb_issue(tb_tile(a, c, t, ntiles), tiles + st * TB_TILE, &S.bar[st], lane);
             }
         issued = g + min(TB_STAGES, ntiles);
-        dd_t acc = dd_zero();
-        for (int t = 0; t < ntiles; ++t) {
+        TbSum acc;
+        const dd_t bc = r < nbc ? ld_dd(a.x + (long)c * TB + r) : dd_zero();
+        bool failed = false; // (the shared word may be set again below: every thread keeps what it saw)
+        for (int t = 0; t < ntiles - 2; ++t) {
             const long gt = g + t;
             const int st = (int)(gt % TB_STAGES);
             const double2 *T = tiles + st * TB_TILE;
-            const bool last = t == ntiles - 1;
             const int p = a.trans == 0 ? t : a.nblk - 1 - t; // block whose x this tile multiplies
-            if (tid == 0) {
-                bool ok = t >= ntiles - 2 || tb_wait_flag(a, p);
-                int code = p + 1; // the block waited for
+            if (tid < TB) {
+                // each lane of warps 0 and 1 waits for an entry of block p
+                bool ok = true;
+                int code = c + 1; // a tile of this block never landed
+                if (tid == 0) ok = tb_wait_bar(&S.bar[st], (uint32_t)((gt / TB_STAGES) & 1), a.wait_ns);
                 if (ok) {
-                    ok = tb_wait_bar(&S.bar[st], (uint32_t)((gt / TB_STAGES) & 1), a.wait_ns);
-                    code = c + 1; // a tile of this block never landed
+                    code = p + 1; // the block waited for
+                    double2 v = make_double2(0.0, 0.0);
+                    if (p * TB + tid < a.n) ok = tb_wait_entry(a, a.xch + ((long)p * TB + tid) * TB_REC, v);
+                    xs[tid] = v;
                 }
                 if (!ok) {
                     S.fail = 1;
@@ -209,58 +304,56 @@ __global__ void __launch_bounds__(TB_THREADS, 1) trsv_blocked_kernel(TbArgs a) {
                 }
             }
             __syncthreads();
-            if (S.fail) break;
-            if (t < ntiles - 2) {
-                const int nbp = min(TB, a.n - p * TB);
-                if (tid < TB) xs[tid] = tid < nbp ? __ldcg(reinterpret_cast<const double2 *>(a.x) + (long)p * TB + tid) : make_double2(0.0, 0.0);
-                __syncthreads();
-                // rows (or columns) r of block c, terms t2 of quarter q
-                const int kn = a.trans == 0 ? TB : nbp;
-                if (r < nbc) {
-                    const int lo = q * 16, hi = min(lo + 16, kn);
-                    if (a.trans == 0) {
-                        for (int t2 = lo; t2 < hi; ++t2) acc = dd_add(acc, dd_mul(sm_dd(T, r + t2 * TB_LD), sm_dd(xs, t2)));
-                    } else {
-                        for (int t2 = lo; t2 < hi; ++t2) acc = dd_add(acc, dd_mul(sm_dd(T, t2 + r * TB_LD), sm_dd(xs, t2)));
-                    }
+            failed = S.fail != 0;
+            if (failed) break;
+            // rows (or columns) r of block c
+            if (r < nbc) tb_dot(acc, T, xs, r, q, 0, a.trans == 0 ? TB : min(TB, a.n - p * TB), a.trans);
+            __syncthreads(); // stage st and xs are free again
+            if (t + TB_STAGES < ntiles) {
+                if (warp == 0) tb_issue(tb_tile(a, c, t + TB_STAGES, ntiles), tiles + st * TB_TILE, &S.bar[st], lane);
+                issued = gt + TB_STAGES + 1;
+            }
+        }
+        if (!failed) {
+            // L(c,c) and W_c
+            const long gl = g + ntiles - 2, gw = gl + 1;
+            const double2 *Lc = tiles + (int)(gl % TB_STAGES) * TB_TILE, *Wc = tiles + (int)(gw % TB_STAGES) * TB_TILE;
+            acc.join();
+            if (tid == TB_THREADS - 1) {
+                const bool ok = tb_wait_bar(&S.bar[gl % TB_STAGES], (uint32_t)((gl / TB_STAGES) & 1), a.wait_ns) &&
+                                tb_wait_bar(&S.bar[gw % TB_STAGES], (uint32_t)((gw / TB_STAGES) & 1), a.wait_ns);
+                if (!ok) {
+                    S.fail = 1;
+                    S.fail_at = gl;
+                    atomicCAS(a.err, 0, c + 1);
                 }
-            } else if (last) {
-                // T = W_c; the previous stage holds L(c,c)
-                const double2 *Lc = tiles + (int)((gt - 1) % TB_STAGES) * TB_TILE;
-                // residual of block c: v = b_c - (sum of the four partial sums)
-                part[q * TB + r] = make_double2(acc.hi, acc.lo);
-                __syncthreads();
-                if (tid < TB) {
-                    dd_t v = dd_zero();
-                    if (tid < nbc) v = dd_sub(ld_dd(a.x + (long)c * TB + tid), tb_sum4(part, tid));
-                    xs[tid] = make_double2(v.hi, v.lo);
-                }
+            }
+            __syncthreads();
+            failed = S.fail != 0;
+            if (!failed) {
+                // v = b_c - the products' sum
+                const dd_t v = r < nbc ? dd_sub(bc, acc.dd()) : dd_zero();
+                if (q == 0) xs[r] = tb_pack(v);
                 __syncthreads();
                 // x0 = W_c v ('N') or W_c^T v ('T')
-                part[q * TB + r] = tb_matvec(T, xs, r, q, nbc, a.trans, false);
-                __syncthreads();
-                if (tid < TB) x0[tid] = tid < nbc ? tb_pack(tb_sum4(part, tid)) : make_double2(0.0, 0.0);
+                const dd_t y = tb_lower(Wc, xs, r, q, nbc, a.trans);
+                if (q == 0) x0[r] = tb_pack(y);
                 __syncthreads();
                 // rs = v - L(c,c) x0 (lower triangle only: the strict upper
                 // part of the tile holds the Schur matrix's own entries)
-                part[q * TB + r] = tb_matvec(Lc, x0, r, q, nbc, a.trans, true);
-                __syncthreads();
-                if (tid < TB) rs[tid] = tid < nbc ? tb_pack(dd_sub(sm_dd(xs, tid), tb_sum4(part, tid))) : make_double2(0.0, 0.0);
+                const dd_t ly = tb_lower(Lc, x0, r, q, nbc, a.trans);
+                if (q == 0) rs[r] = tb_pack(dd_sub(v, ly));
                 __syncthreads();
                 // x = x0 + W_c rs
-                part[q * TB + r] = tb_matvec(T, rs, r, q, nbc, a.trans, false);
-                __syncthreads();
-                if (tid < nbc) st_dd(a.x + (long)c * TB + tid, dd_add(sm_dd(x0, tid), tb_sum4(part, tid)));
-                __threadfence();
+                const dd_t x = dd_add(y, tb_lower(Wc, rs, r, q, nbc, a.trans));
+                if (q == 0 && r < nbc) {
+                    if (c != a.withhold) tb_publish(a.xch + ((long)c * TB + r) * TB_REC, a.epoch, x);
+                    st_dd(a.x + (long)c * TB + r, x);
+                }
+                __syncthreads(); // the stages, xs, x0 and rs are free again
             }
-            __syncthreads(); // stage st and xs are free again
-            if (warp == 0 && t + TB_STAGES < ntiles) {
-                const int sn = (int)((gt + TB_STAGES) % TB_STAGES);
-                tb_issue(tb_tile(a, c, t + TB_STAGES, ntiles), tiles + sn * TB_TILE, &S.bar[sn], lane);
-            }
-            if (t + TB_STAGES < ntiles) issued = gt + TB_STAGES + 1;
         }
-        if (S.fail) {
+        if (failed) {
             // the copies issued but not consumed land (bounded waits)
             // before the CTA exits and its shared memory is reused
             if (tid == 0)
@@ -268,49 +361,53 @@ __global__ void __launch_bounds__(TB_THREADS, 1) trsv_blocked_kernel(TbArgs a) {
             __syncthreads();
             return;
         }
-        if (tid == 0 && c != a.withhold) tb_st_release(a.flags + c, a.epoch);
         g += ntiles;
     }
 }
 
-// W_c = L(c,c)^-1 for every diagonal block: one CTA per block; thread j
-// solves L(c,c) w = e_j for column j (rows j..nb-1, in order, into shared
-// memory), with the reciprocals of the pivots computed once.
+// W_c = L(c,c)^-1 for every diagonal block: one CTA per block; four lanes
+// solve L(c,c) w = e_j for column j (rows j..nb-1, in order, into shared
+// memory), each with every fourth term of a row, with the reciprocals of the
+// pivots computed once.  n = 5003: 60 us; one thread a column 139, and with
+// dd sums 156.
 constexpr size_t TB_INV_SMEM = sizeof(double2) * (2 * (size_t)TB_TILE + TB);
 
-__global__ void __launch_bounds__(TB) trsv_diag_inverse_kernel(const dd_t *L, long lda, int n, dd_t *W) {
+__global__ void __launch_bounds__(TB_THREADS) trsv_diag_inverse_kernel(const dd_t *L, long lda, int n, dd_t *W) {
     extern __shared__ __align__(16) double2 inv_sm[];
     double2 *T = inv_sm;             // L(c,c), lower part
     double2 *Wt = inv_sm + TB_TILE;  // column j of the inverse at Wt + j * TB_LD
     double2 *rp = Wt + TB_TILE;      // 1 / L(i,i)
-    const int c = blockIdx.x, j = threadIdx.x;
+    const int c = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const int j = tb_row(tid >> 5, lane), q = tb_residue(lane);
     const int nb = min(TB, n - c * TB);
     const dd_t *D = L + (long)c * TB + lda * (long)(c * TB);
-    for (int col = 0; col < nb; ++col)
-        if (j < nb && j >= col) T[j + col * TB_LD] = *reinterpret_cast<const double2 *>(D + j + lda * (long)col);
-    __syncthreads();
-    if (j < nb) {
-        const dd_t rj = dd_div(dd_make(1.0, 0.0), sm_dd(T, j + j * TB_LD));
-        rp[j] = make_double2(rj.hi, rj.lo);
+#pragma unroll 4
+    for (int e = tid; e < TB * TB; e += TB_THREADS) {
+        const int i = e % TB, col = e / TB;
+        if (i < nb && col <= i) T[i + col * TB_LD] = *reinterpret_cast<const double2 *>(D + i + lda * (long)col);
     }
     __syncthreads();
+    if (tid < nb) rp[tid] = tb_pack(dd_div(dd_make(1.0, 0.0), sm_dd(T, tid + tid * TB_LD)));
+    __syncthreads();
     double2 *w = Wt + j * TB_LD;
-    if (j < nb) {
-        w[j] = rp[j];
-        for (int i = j + 1; i < nb; ++i) {
-            dd_t s = dd_zero();
-            for (int k = j; k < i; ++k) s = dd_add(s, dd_mul(sm_dd(T, i + k * TB_LD), sm_dd(w, k)));
-            const dd_t v = dd_mul(dd_neg(s), sm_dd(rp, i)); // w_i = -s / L(i,i)
-            w[i] = make_double2(v.hi, v.lo);
-        }
+    if (j < nb && q == 0) w[j] = rp[j];
+    __syncwarp();
+    // a warp's columns go down the rows together
+    for (int i = tb_row(tid >> 5, 0) + 1; i < nb; ++i) {
+        TbSum s;
+#pragma unroll 4
+        for (int k = j + q; k < i; k += TB_Q) s.add(T[i + k * TB_LD], w[k]);
+        s.join();
+        if (i > j && q == 0) w[i] = tb_pack(dd_mul(dd_neg(s.dd()), sm_dd(rp, i))); // w_i = -s / L(i,i)
+        __syncwarp();
     }
     __syncthreads();
     // W_c column-major, leading dimension TB, zero above the diagonal and
     // outside the block; row-coalesced stores
     dd_t *Wc = W + (long)c * TB * TB;
-    for (int col = 0; col < TB; ++col) {
-        const dd_t v = (col < nb && j < nb && j >= col) ? sm_dd(Wt, j + col * TB_LD) : dd_zero();
-        st_dd(Wc + j + (long)TB * col, v);
+    for (int e = tid; e < TB * TB; e += TB_THREADS) {
+        const int i = e % TB, col = e / TB;
+        st_dd(Wc + e, (col < nb && i < nb && i >= col) ? sm_dd(Wt, i + col * TB_LD) : dd_zero());
     }
 }
 
@@ -326,18 +423,18 @@ void trsv_diag_inverse(cudaStream_t st, const dd_t *L, long lda, int n, dd_t *W)
         CK(cudaFuncSetAttribute(trsv_diag_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TB_INV_SMEM));
         attr[dev & 63] = true;
     }
-    trsv_diag_inverse_kernel<<<ceil_div(n, TB), TB, TB_INV_SMEM, st>>>(L, lda, n, W);
+    trsv_diag_inverse_kernel<<<ceil_div(n, TB), TB_THREADS, TB_INV_SMEM, st>>>(L, lda, n, W);
     CK_LAUNCH();
 }
 
-void trsv_blocked(cudaStream_t st, char trans, const dd_t *L, long lda, int n, const dd_t *W, dd_t *x, TrsvSync &sync) {
-    if (n <= 0) return;
+void trsv_blocked(cudaStream_t st, char trans, const dd_t *L, long lda, int n, const dd_t *W, dd_t *x, TrsvSync &sync, int nrhs, long ldx) {
+    if (n <= 0 || nrhs <= 0) return;
     if (trans != 'N' && trans != 'T') throw Error(ERR_ARG, "trsv_blocked: trans must be 'N' or 'T'");
     const int nblk = ceil_div(n, TB);
-    if (nblk > sync.capacity || !sync.flags) throw Error(ERR_ARG, "trsv_blocked: progress flags hold fewer blocks than the solve needs");
+    if ((long)nblk * nrhs > sync.capacity || !sync.xch) throw Error(ERR_ARG, "trsv_blocked: progress flags hold fewer blocks than the solve needs");
     PROF_SCOPE("trsv", st);
     if (++sync.epoch <= 0) sync.epoch = 1;
-    TbArgs a{L, lda, W, n, nblk, sync.epoch, trans == 'N' ? 0 : 1, x, sync.flags, sync.flags + sync.capacity, sync.wait_ns, sync.withhold};
+    TbArgs a{L, lda, W, n, nblk, sync.epoch, trans == 'N' ? 0 : 1, x, sync.xch, sync.flags + sync.capacity, sync.wait_ns, sync.withhold, ldx};
     static thread_local int cap[64] = {};
     int dev = 0;
     CK(cudaGetDevice(&dev));
@@ -350,7 +447,9 @@ void trsv_blocked(cudaStream_t st, char trans, const dd_t *L, long lda, int n, c
         if (per < 1) throw Error(ERR_CUDA, "trsv_blocked: the kernel does not fit on an SM");
         cp = per * sms;
     }
-    const int grid = std::min(nblk, cp);
+    // every CTA of the launch is resident: the right-hand sides share the SMs
+    if (nrhs > cp) throw Error(ERR_ARG, "trsv_blocked: more right-hand sides than resident CTAs");
+    const dim3 grid((unsigned)std::min(nblk, cp / nrhs), (unsigned)nrhs);
     void *args[] = {&a};
     CK(cudaLaunchCooperativeKernel((const void *)trsv_blocked_kernel, grid, TB_THREADS, args, TB_SMEM, st));
     CK_LAUNCH();
