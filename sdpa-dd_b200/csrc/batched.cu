@@ -11,13 +11,14 @@
 // core of all of them as one captured CUDA graph of persistent launches:
 //   zero B                          (bMat.setZero)
 //   F_r = A_r Z^-1, G_r = X F_r     (calF1's two products, one CTA per
-//                                    (problem, constraint, 32 x 32 tile),
+//                                    (problem, constraint, 16 x 16 tile),
 //                                    grid-stride)
 //   B_ij += G_i . A_j, j <= i       (one tiled launch per tile shape, each
 //                                    over the problems assigned to it)
-//   L L^T = B                       (one CTA per problem, right-looking)
+//   L L^T = B                       (after the graph: potrf's block steps,
+//                                    each one launch over all problems)
 // Each entry sees the same operations in the same order as the single-
-// problem kernels (gemm_kernel STORE, schur_dense_pairs_kernel, potrf), so
+// problem kernels (gemm STORE, schur_dense_pairs_kernel, potrf), so
 // every problem's result stays bit for bit that of a single solve.
 //
 // The graph reads a descriptor block (per problem: pointers and sizes; per
@@ -57,16 +58,16 @@ struct CoreItem {
     const dd_t *X, *Zi;
     dd_t *F, *G;            // m n^2 each
     dd_t *B;                // m x m
-    int *info;
 };
 
 struct CoreBatch {
     int count;
     int total_fg;                          // work units of the F and G products
-    int fg_off[CORE_CAP + 1];              // prefix of m * (32 x 32 tiles of n x n)
+    int fg_off[CORE_CAP + 1];              // prefix of m * (16 x 16 tiles of n x n)
     int shape[CORE_CAP];                   // tile shape of each problem
     long tile_off[CORE_SHAPES][CORE_CAP + 1]; // per shape: prefix of its problems' tiles (0 for others)
     CoreItem it[CORE_CAP];
+    PotrfItem pot[CORE_CAP];
 };
 
 // Problem holding flat index u of a prefix array off[0..count] (off[0] = 0).
@@ -93,60 +94,32 @@ __global__ void core_zero_kernel(const CoreBatch *bt) {
 }
 
 // F_r = A_r Z^-1 (stage 0) or G_r = X F_r (stage 1) for every (problem,
-// r): one CTA per 32 x 32 output tile of one product (work units u =
-// fg_off[q] + r * tiles + tile), k in chunks of 16 staged in shared memory,
-// 2 x 2 outputs per thread; every output keeps gemm_kernel's STORE form,
-// acc += Q(k,j) * P(i,k) for k ascending from zero.
-constexpr int FG_T = 32, FG_K = 16;
-__global__ void __launch_bounds__(256) core_fg_kernel(const CoreBatch *bt, int stage) {
-    __shared__ double2 Ps[FG_K][FG_T + 1];
-    __shared__ double2 Qs[FG_K][FG_T + 1];
+// r): one CTA per 16 x 16 output tile of one product (tile16.cuh; work units u
+// = fg_off[q] + r * tiles + tile), every output in gemm's STORE form.  Orders
+// of 10 to 80: larger tiles are mostly padding (a batch of 16 problems of such
+// orders: 354 us a stage on average, in 32 x 32 tiles 528).
+__global__ void __launch_bounds__(T16_THREADS, T16_CTAS) core_fg_kernel(const CoreBatch *bt, int stage) {
+    __shared__ Tile16 S;
     const int total = bt->total_fg;
-    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
     for (int u = blockIdx.x; u < total; u += gridDim.x) {
         const int q = core_find(bt->fg_off, bt->count, u);
         const CoreItem &it = bt->it[q];
-        const int n = it.n, nt = (n + FG_T - 1) / FG_T;
+        const int n = it.n, nt = (n + T16 - 1) / T16;
         const int w = u - bt->fg_off[q], r = w / (nt * nt), tile = w % (nt * nt);
-        const int i0 = (tile % nt) * FG_T, j0 = (tile / nt) * FG_T;
+        const int i0 = (tile % nt) * T16, j0 = (tile / nt) * T16;
         const long nn = (long)n * n;
         const dd_t *P = stage == 0 ? it.A + r * nn : it.X;
         const dd_t *Q = stage == 0 ? it.Zi : it.F + r * nn;
         dd_t *out = stage == 0 ? it.F + r * nn : it.G + r * nn;
-        dd_t acc[2][2] = {{dd_zero(), dd_zero()}, {dd_zero(), dd_zero()}};
-        for (int k0 = 0; k0 < n; k0 += FG_K) {
-            for (int e = tid; e < FG_T * FG_K; e += 256) {
-                const int ii = e % FG_T, kk = e / FG_T;
-                const int gi = i0 + ii, gk = k0 + kk;
-                Ps[kk][ii] = (gi < n && gk < n) ? *reinterpret_cast<const double2 *>(P + gi + (long)n * gk) : make_double2(0.0, 0.0);
-            }
-            for (int e = tid; e < FG_T * FG_K; e += 256) {
-                const int kk = e % FG_K, jj = e / FG_K;
-                const int gj = j0 + jj, gk = k0 + kk;
-                Qs[kk][jj] = (gj < n && gk < n) ? *reinterpret_cast<const double2 *>(Q + gk + (long)n * gj) : make_double2(0.0, 0.0);
-            }
-            __syncthreads();
-            const int kmax = min(FG_K, n - k0);
-            for (int kk = 0; kk < kmax; ++kk) {
-                dd_t a[2], b[2];
+        dd_t acc[2] = {dd_zero(), dd_zero()};
+        tile16_sum<false, true, false, false>(
+            S, n, [&](int i, long k) { return i0 + i < n ? *reinterpret_cast<const double2 *>(P + i0 + i + n * k) : make_double2(0.0, 0.0); },
+            [&](int j, long k) { return j0 + j < n ? *reinterpret_cast<const double2 *>(Q + k + (long)n * (j0 + j)) : make_double2(0.0, 0.0); }, acc);
 #pragma unroll
-                for (int x = 0; x < 2; ++x) a[x] = dd_make(Ps[kk][ty + 16 * x].x, Ps[kk][ty + 16 * x].y);
-#pragma unroll
-                for (int y = 0; y < 2; ++y) b[y] = dd_make(Qs[kk][tx + 16 * y].x, Qs[kk][tx + 16 * y].y);
-#pragma unroll
-                for (int x = 0; x < 2; ++x)
-#pragma unroll
-                    for (int y = 0; y < 2; ++y) acc[x][y] = dd_acc(acc[x][y], dd_mul(b[y], a[x]));
-            }
-            __syncthreads();
+        for (int x = 0; x < 2; ++x) {
+            const int i = i0 + threadIdx.x / T16 + 8 * x, j = j0 + threadIdx.x % T16;
+            if (i < n && j < n) st_dd(out + i + (long)n * j, acc[x]);
         }
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-#pragma unroll
-            for (int y = 0; y < 2; ++y) {
-                const int i = i0 + ty + 16 * x, j = j0 + tx + 16 * y;
-                if (i < n && j < n) st_dd(out + i + (long)n * j, acc[x][y]);
-            }
     }
 }
 
@@ -250,66 +223,6 @@ __global__ void __launch_bounds__(T16_THREADS, T16_CTAS) core_pairs16_kernel(con
     }
 }
 
-// In-place lower Cholesky of every problem's B, one CTA per problem,
-// right-looking column by column: pivot (sqrt, then the reciprocal
-// 1/L(j,j)), scaling of the column by it, then the update of the trailing
-// lower triangle; every entry takes x - L(j,k) L(i,k) for k ascending and
-// then its sqrt or scaling, as potrf's kernels do.  *info: the 1-based
-// failing column.
-constexpr int CORE_POTRF_THREADS = 1024;
-__global__ void __launch_bounds__(CORE_POTRF_THREADS) core_potrf_kernel(const CoreBatch *bt) {
-    const int q = blockIdx.x;
-    if (q >= bt->count) return;
-    const CoreItem &it = bt->it[q];
-    const int m = it.m;
-    dd_t *A = it.B;
-    __shared__ double2 rj;
-    __shared__ int fail;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    if (tid == 0) fail = 0;
-    __syncthreads();
-    for (int j = 0; j < m; ++j) {
-        if (tid == 0) {
-            const dd_t d = ld_dd(A + j + (long)m * j);
-            if (dd_le_d(d, 0.0) || dd_isnan(d)) {
-                fail = 1;
-                *it.info = j + 1;
-            } else {
-                const dd_t l = dd_sqrt(d);
-                st_dd(A + j + (long)m * j, l);
-                const dd_t r = dd_div(dd_from(1.0), l);
-                rj = make_double2(r.hi, r.lo);
-            }
-        }
-        __syncthreads();
-        if (fail) return;
-        const dd_t r = dd_make(rj.x, rj.y);
-        for (int i = j + 1 + tid; i < m; i += nt) st_dd(A + i + (long)m * j, dd_mul(r, ld_dd(A + i + (long)m * j)));
-        __syncthreads();
-        // trailing lower triangle: entries (i, k), j < k <= i
-        const int w = m - j - 1;
-        const long cnt = (long)w * (w + 1) / 2;
-        for (long e = tid; e < cnt; e += nt) {
-            // e -> (k, i): column k = j+1+c, rows i = k..m-1; column-major packing
-            const int c = (int)((2.0 * w + 1.0 - sqrt((2.0 * w + 1.0) * (2.0 * w + 1.0) - 8.0 * (double)e)) / 2.0);
-            int cc = c;
-            long base = (long)cc * w - (long)cc * (cc - 1) / 2;
-            while (base > e) { // guard the floating estimate
-                --cc;
-                base = (long)cc * w - (long)cc * (cc - 1) / 2;
-            }
-            while (base + (w - cc) <= e) {
-                base += w - cc;
-                ++cc;
-            }
-            const int k = j + 1 + cc, i = k + (int)(e - base);
-            dd_t *p = A + i + (long)m * k;
-            st_dd(p, dd_sub(ld_dd(p), dd_mul(ld_dd(A + k + (long)m * j), ld_dd(A + i + (long)m * j))));
-        }
-        __syncthreads();
-    }
-}
-
 struct Shape {
     int bm, bn;
 };
@@ -366,8 +279,8 @@ CoreEngine::CoreEngine(int device) : p(new Impl) {
     CK(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
     cudaMemcpyAsync(p->db, p->hb, sizeof(CoreBatch), cudaMemcpyHostToDevice, p->stream);
     core_zero_kernel<<<dim3(8, CORE_CAP), 256, 0, p->stream>>>(p->db);
-    core_fg_kernel<<<4 * p->sms, 256, 0, p->stream>>>(p->db, 0);
-    core_fg_kernel<<<4 * p->sms, 256, 0, p->stream>>>(p->db, 1);
+    core_fg_kernel<<<8 * p->sms, T16_THREADS, 0, p->stream>>>(p->db, 0);
+    core_fg_kernel<<<8 * p->sms, T16_THREADS, 0, p->stream>>>(p->db, 1);
     cudaEventRecordWithFlags(p->ev_shape[0][0], p->stream, cudaEventRecordExternal);
     core_pairs16_kernel<<<8 * p->sms, T16_THREADS, 0, p->stream>>>(p->db);
     cudaEventRecordWithFlags(p->ev_shape[0][1], p->stream, cudaEventRecordExternal);
@@ -377,7 +290,6 @@ CoreEngine::CoreEngine(int device) : p(new Impl) {
     cudaEventRecordWithFlags(p->ev_shape[2][0], p->stream, cudaEventRecordExternal);
     core_pairs_kernel<2, 64, 64, 16, 4, 4><<<2 * p->sms, 256, 0, p->stream>>>(p->db);
     cudaEventRecordWithFlags(p->ev_shape[2][1], p->stream, cudaEventRecordExternal);
-    core_potrf_kernel<<<CORE_CAP, CORE_POTRF_THREADS, 0, p->stream>>>(p->db);
     cudaError_t cap = cudaStreamEndCapture(p->stream, &g);
     if (cap != cudaSuccess) throw Error(ERR_CUDA, std::string("batched core: graph capture failed: ") + cudaGetErrorString(cap));
     CK(cudaGraphInstantiate(&p->exec, g, 0));
@@ -431,6 +343,7 @@ void CoreEngine::launch_locked() {
     for (int s = 0; s < CORE_SHAPES; ++s) b.tile_off[s][0] = 0;
     double terms[CORE_SHAPES] = {0, 0, 0};
     int cls_of_shape[CORE_SHAPES] = {-1, -1, -1};
+    int mmax = 0;
     for (int q = 0; q < cnt; ++q) {
         Context &c = *I.pending[q];
         const BlockDev &bd = *c.blocks[0];
@@ -445,8 +358,9 @@ void CoreEngine::launch_locked() {
         it.F = c.Fbuf.p;
         it.G = c.Gbuf.p;
         it.B = c.B.p;
-        it.info = c.info.p;
-        const int ntl = (bd.n + 31) / 32;
+        b.pot[q] = {c.B.p, c.rdiag.p, c.info.p, c.m};
+        mmax = std::max(mmax, c.m);
+        const int ntl = (bd.n + T16 - 1) / T16;
         b.fg_off[q + 1] = b.fg_off[q] + c.m * ntl * ntl;
         const int cl = size_class(c.m);
         const int s = cls_shape[cl];
@@ -467,6 +381,7 @@ void CoreEngine::launch_locked() {
     }
     b.total_fg = b.fg_off[cnt];
     CK(cudaGraphLaunch(I.exec, I.stream));
+    potrf_list(I.stream, I.db->pot, cnt, mmax);
     CK(cudaEventRecord(I.done, I.stream));
     for (int q = 0; q < cnt; ++q) CK(cudaStreamWaitEvent(I.pending[q]->stream, I.done, 0));
     // autotuner: time the shapes this batch measured (one class each)

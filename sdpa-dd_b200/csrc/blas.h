@@ -39,6 +39,14 @@ void zero_upper(cudaStream_t st, dd_t *A, long lda, int n, int batch = 1, long s
 // one CTA each (the single diagonal block of potrf); any failure sets
 // *info_dev to a failing column.
 void potrf_batched(cudaStream_t st, dd_t *A, long lda, int n, long sA, int batch, int *info_dev);
+// Rpotrf("Lower") of `count` matrices of orders up to nmax (a list in device
+// memory; leading dimension n, rdiag room for 64 reciprocals, info zero).
+struct PotrfItem {
+    dd_t *A, *rdiag;
+    int *info;
+    int n;
+};
+void potrf_list(cudaStream_t st, const PotrfItem *list_dev, int count, int nmax);
 // Progress words of the one-launch triangular solve: one flag per 64-entry
 // block (the epoch of the solve that finished it), then an error word; and
 // the blocked solves' published entries, with the epoch beside them.
