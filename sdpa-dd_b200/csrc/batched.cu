@@ -23,8 +23,9 @@
 //
 // The graph reads a descriptor block (per problem: pointers and sizes; per
 // tile shape: the prefix of its tiles) that the engine copies from pinned
-// memory as the graph's first node, so one instantiated graph serves every
-// batch whatever its problems.
+// memory before it, so one instantiated graph serves every batch whatever its
+// problems.  The copy waits for the batch's own streams, so the pinned blocks
+// take turns, and one is written again only when its last copy is done.
 //
 // Tile shapes of the pair products are picked per size class of m by a
 // small autotuner: the first batches of a class time each candidate shape
@@ -46,6 +47,7 @@ namespace sddd {
 namespace {
 
 constexpr int CORE_CAP = 256;      // problems per batch
+constexpr int CORE_RING = 4;       // descriptor blocks in pinned memory, in turn
 constexpr int CORE_SHAPES = 3;     // candidate tile shapes of the pair products
 constexpr int CORE_MAX_M = 1024;
 constexpr int CORE_MAX_N = 128;
@@ -237,7 +239,9 @@ struct CoreEngine::Impl {
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
     cudaEvent_t ev_shape[CORE_SHAPES][2] = {};
-    CoreBatch *hb = nullptr, *db = nullptr;
+    CoreBatch *hb = nullptr, *db = nullptr; // hb: CORE_RING blocks
+    cudaEvent_t copied[CORE_RING] = {};
+    int turn = 0;
     cudaGraphExec_t exec = nullptr;
     int sms = 148;
     // autotuner: per size class, the chosen shape (-1: still measuring) and
@@ -264,20 +268,20 @@ CoreEngine::CoreEngine(int device) : p(new Impl) {
         CK(cudaEventCreate(&e[0]));
         CK(cudaEventCreate(&e[1]));
     }
-    CK(cudaMallocHost(&p->hb, sizeof(CoreBatch)));
+    for (auto &e : p->copied) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    CK(cudaMallocHost(&p->hb, CORE_RING * sizeof(CoreBatch)));
     CK(cudaMalloc(&p->db, sizeof(CoreBatch)));
-    std::memset(p->hb, 0, sizeof(CoreBatch));
+    std::memset(p->hb, 0, CORE_RING * sizeof(CoreBatch));
     CK(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, device));
     for (auto &row : p->per_term)
         for (double &v : row) v = -1.0;
-    // the graph: descriptor copy, zero, F, G, the pair products of each
+    // the graph: zero, F, G, the pair products of each
     // shape between event-record nodes (recorded as external events, so
     // that every launch of the graph records them and the autotuner can
     // time the shapes; a plain record inside a capture only orders the
     // graph), the factorisations
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
-    cudaMemcpyAsync(p->db, p->hb, sizeof(CoreBatch), cudaMemcpyHostToDevice, p->stream);
     core_zero_kernel<<<dim3(8, CORE_CAP), 256, 0, p->stream>>>(p->db);
     core_fg_kernel<<<8 * p->sms, T16_THREADS, 0, p->stream>>>(p->db, 0);
     core_fg_kernel<<<8 * p->sms, T16_THREADS, 0, p->stream>>>(p->db, 1);
@@ -305,6 +309,7 @@ CoreEngine::~CoreEngine() {
         cudaEventDestroy(e[1]);
     }
     cudaEventDestroy(p->done);
+    for (auto &e : p->copied) cudaEventDestroy(e);
     cudaStreamDestroy(p->stream);
     cudaFreeHost(p->hb);
     cudaFree(p->db);
@@ -326,7 +331,9 @@ void CoreEngine::leave() {
 // Runs under mu: the pending problems as one graph launch.
 void CoreEngine::launch_locked() {
     Impl &I = *p;
-    CoreBatch &b = *I.hb;
+    I.turn = (I.turn + 1) % CORE_RING;
+    CK(cudaEventSynchronize(I.copied[I.turn]));
+    CoreBatch &b = I.hb[I.turn];
     const int cnt = (int)I.pending.size();
     // the shape of each problem: its class's choice, or (while the class is
     // measured) the next candidate it has not timed
@@ -380,6 +387,8 @@ void CoreEngine::launch_locked() {
         CK(cudaStreamWaitEvent(I.stream, c.core_ready, 0));
     }
     b.total_fg = b.fg_off[cnt];
+    CK(cudaMemcpyAsync(I.db, &b, sizeof(CoreBatch), cudaMemcpyHostToDevice, I.stream));
+    CK(cudaEventRecord(I.copied[I.turn], I.stream));
     CK(cudaGraphLaunch(I.exec, I.stream));
     potrf_list(I.stream, I.db->pot, cnt, mmax);
     CK(cudaEventRecord(I.done, I.stream));
