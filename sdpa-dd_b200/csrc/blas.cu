@@ -357,22 +357,10 @@ __device__ __forceinline__ bool bar_wait0(uint64_t *b) {
         if (globaltimer_ns() - t0 > POTRF_WAIT_NS) return false;
     return true;
 }
-// list: CTA b takes matrix b of a list (potrf_list), its block at column c0.
-__global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_kernel(dd_t *A, long lda, int nb, int c0, int *info, dd_t *rdiag, long sA,
-                                                                  const PotrfItem *list) {
+__device__ __forceinline__ void potrf_diag_body(dd_t *A, long lda, int nb, int c0, int *info, dd_t *rdiag) {
     extern __shared__ double2 sm[];
-    if (list) {
-        const PotrfItem &it = list[blockIdx.x];
-        if (c0 >= it.n) return;
-        A = it.A;
-        lda = it.n;
-        nb = min(POTRF_NB, it.n - c0);
-        info = it.info;
-        rdiag = it.rdiag;
-    }
     double2 *S = sm; // nb x nb, column-major: columns on their way, then final
     __shared__ int stop; // k + 1: bad pivot k
-    if (!list) A += blockIdx.x * sA; // CTA b: matrix b of a batch of equal blocks (rdiag null then)
     if (*info != 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) stop = 0;
@@ -491,6 +479,17 @@ __global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_kernel(dd_t *A, long 
         const int i = e % nb, j = e / nb;
         if (i >= j) st_dd(A + (c0 + i) + lda * (long)(c0 + j), at(i, j));
     }
+}
+
+// CTA b: matrix b of a batch of equal blocks (rdiag null then).
+__global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_kernel(dd_t *A, long lda, int nb, int c0, int *info, dd_t *rdiag, long sA) {
+    potrf_diag_body(A + blockIdx.x * sA, lda, nb, c0, info, rdiag);
+}
+// CTA b: the block at column c0 of matrix b of a list (a kernel of its own:
+// with the block's order and pointers in registers it takes 66 us, not 48).
+__global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_list_kernel(const PotrfItem *list, int c0) {
+    const PotrfItem &it = list[blockIdx.x];
+    if (c0 < it.n) potrf_diag_body(it.A, it.n, min(POTRF_NB, it.n - c0), c0, it.info, it.rdiag);
 }
 
 // Panel rows below the diagonal block (Rtrsm "Right", "Lower", "Transpose":
@@ -670,7 +669,7 @@ void potrf(cudaStream_t st, dd_t *A, long lda, int n, int *info_dev, dd_t *rdiag
         // block) runs; panel k+1 waits for both.
         {
             PROF_SCOPE("potrf_diag", st);
-            potrf_diag_kernel<<<1, DIAG_THREADS, sizeof(double2) * nbmax * nbmax, st>>>(A, lda, nbmax, 0, info_dev, rdiag_dev, 0, nullptr);
+            potrf_diag_kernel<<<1, DIAG_THREADS, sizeof(double2) * nbmax * nbmax, st>>>(A, lda, nbmax, 0, info_dev, rdiag_dev, 0);
             CK_LAUNCH();
         }
         for (int c0 = 0;; c0 += nbmax) {
@@ -692,7 +691,7 @@ void potrf(cudaStream_t st, dd_t *A, long lda, int n, int *info_dev, dd_t *rdiag
             CK(cudaStreamWaitEvent(tc->side, tc->ev_pre, 0));
             {
                 PROF_SCOPE("potrf_diag", tc->side);
-                potrf_diag_kernel<<<1, DIAG_THREADS, sizeof(double2) * nb1 * nb1, tc->side>>>(A, lda, nb1, c1, info_dev, rdiag_dev, 0, nullptr);
+                potrf_diag_kernel<<<1, DIAG_THREADS, sizeof(double2) * nb1 * nb1, tc->side>>>(A, lda, nb1, c1, info_dev, rdiag_dev, 0);
                 CK_LAUNCH();
             }
             CK(cudaEventRecord(tc->ev_diag, tc->side));
@@ -708,7 +707,7 @@ void potrf(cudaStream_t st, dd_t *A, long lda, int n, int *info_dev, dd_t *rdiag
         const int nb = std::min(nbmax, n - c0);
         {
             PROF_SCOPE("potrf_diag", st);
-            potrf_diag_kernel<<<1, DIAG_THREADS, sizeof(double2) * nb * nb, st>>>(A, lda, nb, c0, info_dev, rdiag_dev, 0, nullptr);
+            potrf_diag_kernel<<<1, DIAG_THREADS, sizeof(double2) * nb * nb, st>>>(A, lda, nb, c0, info_dev, rdiag_dev, 0);
             CK_LAUNCH();
         }
         const int below = n - c0 - nb;
@@ -740,7 +739,7 @@ void potrf_batched(cudaStream_t st, dd_t *A, long lda, int n, long sA, int batch
     if (n > POTRF_NB) throw Error(ERR_ARG, "potrf_batched: order above one diagonal block");
     const size_t smem = sizeof(double2) * n * n;
     CK(cudaFuncSetAttribute(potrf_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(double2) * POTRF_NB * POTRF_NB)));
-    potrf_diag_kernel<<<batch, DIAG_THREADS, smem, st>>>(A, lda, n, 0, info_dev, nullptr, sA, nullptr);
+    potrf_diag_kernel<<<batch, DIAG_THREADS, smem, st>>>(A, lda, n, 0, info_dev, nullptr, sA);
     CK_LAUNCH();
 }
 
@@ -782,10 +781,10 @@ void potrf_list(cudaStream_t st, const PotrfItem *list_dev, int count, int nmax)
     if (count <= 0 || nmax <= 0) return;
     if (count > MAX_GRID_YZ) throw Error(ERR_ARG, "potrf_list: more matrices than a grid row holds");
     const size_t smem = sizeof(double2) * POTRF_NB * POTRF_NB;
-    CK(cudaFuncSetAttribute(potrf_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaFuncSetAttribute(potrf_diag_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CK(cudaFuncSetAttribute(potrf_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM));
     for (int c0 = 0; c0 < nmax; c0 += POTRF_NB) {
-        potrf_diag_kernel<<<count, DIAG_THREADS, smem, st>>>(nullptr, 0, 0, c0, nullptr, nullptr, 0, list_dev);
+        potrf_diag_list_kernel<<<count, DIAG_THREADS, smem, st>>>(list_dev, c0);
         CK_LAUNCH();
         const int below = nmax - c0 - POTRF_NB;
         if (below <= 0) break;
