@@ -357,7 +357,9 @@ __device__ __forceinline__ bool bar_wait0(uint64_t *b) {
         if (globaltimer_ns() - t0 > POTRF_WAIT_NS) return false;
     return true;
 }
-__device__ __forceinline__ void potrf_diag_body(dd_t *A, long lda, int nb, int c0, int *info, dd_t *rdiag) {
+template <int NB>
+__device__ __forceinline__ void potrf_diag_body(dd_t *A, long lda, int nb_, int c0, int *info, dd_t *rdiag) {
+    const int nb = NB > 0 ? NB : nb_;
     extern __shared__ double2 sm[];
     double2 *S = sm; // nb x nb, column-major: columns on their way, then final
     __shared__ int stop; // k + 1: bad pivot k
@@ -483,13 +485,14 @@ __device__ __forceinline__ void potrf_diag_body(dd_t *A, long lda, int nb, int c
 
 // CTA b: matrix b of a batch of equal blocks (rdiag null then).
 __global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_kernel(dd_t *A, long lda, int nb, int c0, int *info, dd_t *rdiag, long sA) {
-    potrf_diag_body(A + blockIdx.x * sA, lda, nb, c0, info, rdiag);
+    if (nb == POTRF_NB) potrf_diag_body<POTRF_NB>(A + blockIdx.x * sA, lda, nb, c0, info, rdiag);
+    else potrf_diag_body<0>(A + blockIdx.x * sA, lda, nb, c0, info, rdiag);
 }
 // CTA b: the block at column c0 of matrix b of a list (a kernel of its own:
 // with the block's order and pointers in registers it takes 66 us, not 48).
 __global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_list_kernel(const PotrfItem *list, int c0) {
     const PotrfItem &it = list[blockIdx.x];
-    if (c0 < it.n) potrf_diag_body(it.A, it.n, min(POTRF_NB, it.n - c0), c0, it.info, it.rdiag);
+    if (c0 < it.n) potrf_diag_body<0>(it.A, it.n, min(POTRF_NB, it.n - c0), c0, it.info, it.rdiag);
 }
 
 // Panel rows below the diagonal block (Rtrsm "Right", "Lower", "Transpose":
