@@ -497,32 +497,37 @@ __global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_list_kernel(const Pot
 
 // Panel rows below the diagonal block (Rtrsm "Right", "Lower", "Transpose":
 // x(i,j) -= L(j,k) x(i,k) for k < j ascending, then x(i,j) *= 1/L(j,j)).
-// Rows are independent, so a warp solves PANEL_WROWS rows by itself, with
-// no barrier: lane = (column class c, row r), c = lane / PANEL_WROWS, and
-// the lane holds the row's columns c, c + PANEL_CLASSES, ... in registers.
-// At step k the holder of x(r,k) passes it to the row's other lanes by
-// shuffle; every lane subtracts the step's term from its columns right of
-// k, and the holder of column k + 1 then scales it (the entry is final).
-// Rounds of PANEL_CLASSES steps: in round q, slot s holds column
-// c + PANEL_CLASSES (q + s) (the slots rotate by one between rounds, and the
-// column leaving slot 0 is final and goes back to memory); the rounds are
-// unrolled so that each one updates exactly its live slots, without
-// branches between the slots' independent chains.  L11 (lower triangle,
-// packed by columns, one bulk copy per column) and the reciprocals are
-// shared by the CTA's warps.  The panel is POTRF_NB columns wide.
-constexpr int PANEL_CLASSES = 16;                           // lanes a row
-constexpr int PANEL_WROWS = 32 / PANEL_CLASSES;             // rows a warp
-constexpr int PANEL_SLOTS = POTRF_NB / PANEL_CLASSES;       // columns a lane
+// Rows are independent, so a warp solves W = 32 / C rows by itself, with no
+// barrier: lane = (column class c, row r), c = lane / W, and the lane holds the
+// row's columns c, c + C, ... in registers.  At step k the holder of x(r,k)
+// passes it to the row's other lanes by shuffle; every lane scales it (the
+// entry is final; no branch for its holder) and subtracts the step's term from
+// its columns right of k.
+// Rounds of C steps: in round q, slot s holds column c + C (q + s) (the slots
+// rotate by one between rounds, and the column leaving slot 0 is final and goes
+// back to memory); the rounds are unrolled so that each one updates exactly its
+// live slots, without branches between the slots' independent chains.  L11
+// (lower triangle, packed by columns, one bulk copy per column) and the
+// reciprocals are shared by the CTA's warps.  The panel is POTRF_NB columns
+// wide.
+// A step is a shuffle, a product, and a product and a subtraction (190
+// cycles), or the FP64 issue of the live slots where there are rows enough.
+// Measured (C = 16 / 8): 500 rows 14.0 / 15.4 us, 1500 16.9 / 15.8, 5000 35 /
+// 31, 10000 58 / 48.6; with the holder scaling its entry under a branch and C =
+// 16 18.5, 20.8, 37.5 and 60.
 constexpr int PANEL_THREADS = 128;
-constexpr int PANEL_ROWS = PANEL_WROWS * (PANEL_THREADS / 32); // rows a CTA
-static_assert(POTRF_NB % PANEL_CLASSES == 0 && 32 % PANEL_CLASSES == 0, "panel lane map");
+// lanes a row -> rows a CTA
+__host__ __device__ constexpr int panel_rows(int classes) { return 32 / classes * (PANEL_THREADS / 32); }
 constexpr size_t PANEL_SMEM = sizeof(double2) * (POTRF_NB * (POTRF_NB + 1) / 2 + POTRF_NB);
 // first entry of column k (rows k .. POTRF_NB-1) of a lower triangle packed
 // by columns
 __device__ __forceinline__ int col_off(int k) { return k * POTRF_NB - k * (k - 1) / 2; }
+template <int PANEL_CLASSES>
 __global__ void __launch_bounds__(PANEL_THREADS) potrf_panel_kernel(dd_t *A, long lda, int n, int c0, int *info, const dd_t *rdiag,
                                                                     const PotrfItem *list) {
-    constexpr int NB = POTRF_NB, C = PANEL_CLASSES, W = PANEL_WROWS, NS = PANEL_SLOTS;
+    // lanes and columns a lane a row, rows a warp and a CTA
+    constexpr int NB = POTRF_NB, C = PANEL_CLASSES, W = 32 / C, NS = NB / C, PANEL_ROWS = panel_rows(C);
+    static_assert(NB % C == 0 && 32 % C == 0, "panel lane map");
     extern __shared__ __align__(16) double2 sm[];
     double2 *L11 = sm;                   // lower triangle of NB x NB, packed by columns
     double2 *R = sm + NB * (NB + 1) / 2; // NB reciprocals
@@ -568,34 +573,25 @@ __global__ void __launch_bounds__(PANEL_THREADS) potrf_panel_kernel(dd_t *A, lon
     __syncthreads();
     if (lfail) return;
     auto rk = [&](int k) { return dd_make(R[k].x, R[k].y); };
-    if (cls == 0) x[0] = dd_mul(rk(0), x[0]); // column 0: scaling only
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
         // step k = C q + t; slot s holds column cls + C (q + s), s < NS - q
 #pragma unroll 1
         for (int t = 0; t < C; ++t) {
             const int k = C * q + t;
-            if (k + 1 >= NB) break;
-            const dd_t xk = dd_make(__shfl_sync(0xffffffffu, x[0].hi, t * W + row), __shfl_sync(0xffffffffu, x[0].lo, t * W + row));
             const double2 *lk = L11 + col_off(k) - k; // L(j, k) at lk[j]
+            // x(r,k), final after its scaling, in all the row's lanes
+            const dd_t xk = dd_mul(rk(k), dd_make(__shfl_sync(0xffffffffu, x[0].hi, t * W + row), __shfl_sync(0xffffffffu, x[0].lo, t * W + row)));
             dd_t y[NS];
 #pragma unroll
             for (int s = 0; s < NS - q; ++s) {
-                const int j = cls + C * (q + s);
-                const double2 l = lk[j];
+                // (slot 0's columns left of k read some entry of L11, unused)
+                const double2 l = lk[s == 0 ? max(cls + C * q, k) : cls + C * (q + s)];
                 y[s] = dd_sub(x[s], dd_mul(dd_make(l.x, l.y), xk));
             }
-            // slot 0's column lies right of k only for classes above t
-            x[0] = cls > t ? y[0] : x[0];
+            x[0] = cls > t ? y[0] : cls == t ? xk : x[0];
 #pragma unroll
             for (int s = 1; s < NS - q; ++s) x[s] = y[s];
-            // column k + 1 is final after its scaling: class t + 1 in slot 0,
-            // or class 0 in slot 1 at the round's last step
-            if (t + 1 < C) {
-                if (cls == t + 1) x[0] = dd_mul(rk(k + 1), x[0]);
-            } else if (q + 1 < NS) {
-                if (cls == 0) x[1] = dd_mul(rk(k + 1), x[1]);
-            }
         }
         // column cls + C q is final
         if (live) st_dd(arow + lda * (long)(cls + C * q), x[0]);
@@ -646,6 +642,23 @@ __global__ void potrf_diag_pre_kernel(dd_t *A, long lda, int c0, int nb, int nbp
     st_dd(d, x);
 }
 
+static void panel_attr() {
+    CK(cudaFuncSetAttribute(potrf_panel_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM));
+    CK(cudaFuncSetAttribute(potrf_panel_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM));
+}
+// `below` rows of each of `count` matrices.  Few rows: 16 lanes a row keep a
+// step's chain short; more rows than fill the SM sub-partitions (two rows a
+// warp): 8 lanes, whose slots idle less.  1000 rows 14.3 us with 16, 15.6 with
+// 8; 1500 rows 16.9 and 15.8.
+constexpr long PANEL_FEW_ROWS = 1184;
+static void panel_launch(cudaStream_t st, dd_t *A, long lda, int n, int c0, int below, int count, int *info, const dd_t *rdiag, const PotrfItem *list) {
+    const long rows = (long)below * count;
+    auto grid = [&](int c) { return dim3((unsigned)ceil_div(below, panel_rows(c)), (unsigned)count); };
+    if (rows <= PANEL_FEW_ROWS) potrf_panel_kernel<16><<<grid(16), PANEL_THREADS, PANEL_SMEM, st>>>(A, lda, n, c0, info, rdiag, list);
+    else potrf_panel_kernel<8><<<grid(8), PANEL_THREADS, PANEL_SMEM, st>>>(A, lda, n, c0, info, rdiag, list);
+    CK_LAUNCH();
+}
+
 // Right-looking blocked Cholesky: per panel of POTRF_NB columns, factor the
 // diagonal block, solve the rows below, then subtract the panel's outer
 // product from the trailing lower triangle (GEMM_SUB keeps each entry's
@@ -655,12 +668,11 @@ void potrf(cudaStream_t st, dd_t *A, long lda, int n, int *info_dev, dd_t *rdiag
     static thread_local bool attr[64] = {};
     const int nbmax = POTRF_NB;
     const size_t smem_diag = sizeof(double2) * nbmax * nbmax;
-    const size_t smem_panel = PANEL_SMEM;
     int dev = 0;
     CK(cudaGetDevice(&dev));
     if (!attr[dev & 63]) {
         CK(cudaFuncSetAttribute(potrf_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_diag));
-        CK(cudaFuncSetAttribute(potrf_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_panel));
+        panel_attr();
         CK(cudaFuncSetAttribute(potrf_diag_pre_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(double2) * nbmax * nbmax)));
         attr[dev & 63] = true;
     }
@@ -681,8 +693,7 @@ void potrf(cudaStream_t st, dd_t *A, long lda, int n, int *info_dev, dd_t *rdiag
             if (below <= 0) break;
             {
                 PROF_SCOPE("potrf_panel", st);
-                potrf_panel_kernel<<<ceil_div(below, PANEL_ROWS), PANEL_THREADS, PANEL_SMEM, st>>>(A, lda, n, c0, info_dev, rdiag_dev, nullptr);
-                CK_LAUNCH();
+                panel_launch(st, A, lda, n, c0, below, 1, info_dev, rdiag_dev, nullptr);
             }
             const int c1 = c0 + nb, nb1 = std::min(nbmax, n - c1);
             {
@@ -717,8 +728,7 @@ void potrf(cudaStream_t st, dd_t *A, long lda, int n, int *info_dev, dd_t *rdiag
         if (below <= 0) break;
         {
             PROF_SCOPE("potrf_panel", st);
-            potrf_panel_kernel<<<ceil_div(below, PANEL_ROWS), PANEL_THREADS, PANEL_SMEM, st>>>(A, lda, n, c0, info_dev, rdiag_dev, nullptr);
-            CK_LAUNCH();
+            panel_launch(st, A, lda, n, c0, below, 1, info_dev, rdiag_dev, nullptr);
         }
         dd_t *panel = A + (c0 + nb) + lda * (long)c0;
         dd_t *trail = A + (c0 + nb) + lda * (long)(c0 + nb);
@@ -785,14 +795,13 @@ void potrf_list(cudaStream_t st, const PotrfItem *list_dev, int count, int nmax)
     if (count > MAX_GRID_YZ) throw Error(ERR_ARG, "potrf_list: more matrices than a grid row holds");
     const size_t smem = sizeof(double2) * POTRF_NB * POTRF_NB;
     CK(cudaFuncSetAttribute(potrf_diag_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaFuncSetAttribute(potrf_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM));
+    panel_attr();
     for (int c0 = 0; c0 < nmax; c0 += POTRF_NB) {
         potrf_diag_list_kernel<<<count, DIAG_THREADS, smem, st>>>(list_dev, c0);
         CK_LAUNCH();
         const int below = nmax - c0 - POTRF_NB;
         if (below <= 0) break;
-        potrf_panel_kernel<<<dim3(ceil_div(below, PANEL_ROWS), count), PANEL_THREADS, PANEL_SMEM, st>>>(nullptr, 0, 0, c0, nullptr, nullptr, list_dev);
-        CK_LAUNCH();
+        panel_launch(st, nullptr, 0, 0, c0, below, count, nullptr, nullptr, list_dev);
         const long nt = ceil_div(below, T16), tiles = nt * (nt + 1) / 2;
         const dim3 grid((unsigned)tiles, count);
         if (tiles * count <= T16_PIPE_TILES)
