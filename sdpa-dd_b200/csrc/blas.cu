@@ -1199,6 +1199,79 @@ __global__ void __launch_bounds__(INV_THREADS) inv_lower_small_kernel(const dd_t
     for (int i = tid; i < n; i += INV_THREADS) *reinterpret_cast<double2 *>(X + i + ldx * (long)j) = col[i];
 }
 
+// The same for n <= 32 NW R with a column in registers: thread t holds rows j +
+// t + 32 NW r.  A step's chain, a quotient (the reciprocals of the diagonal
+// formed beforehand, fastdiv.cuh), a product and a subtraction, runs in every
+// thread on the next entry, which the step before broadcast without its last
+// term, so that the barrier of a step is not in the chain; L's entries are
+// loaded two steps ahead.
+// Measured, n = 500: 318 us; with the quotient on one thread between two
+// barriers and L's column read when it is needed 540.  Up to 256 rows the form
+// above is the faster one (n = 150: 36 us, this 46; n = 20: 7 and 10): its
+// quotient costs one warp's issue slots, here every warp's.
+template <int NW, int R>
+__global__ void __launch_bounds__(32 * NW) inv_lower_rows_kernel(const dd_t *L, long lda, int n, dd_t *X, long ldx, long sL, long sX) {
+    constexpr int T = 32 * NW;
+    extern __shared__ double2 inv_sm[];
+    double2 *dg = inv_sm, *sd = dg + n; // L(k,k), L(k+1,k)
+    double *rc = reinterpret_cast<double *>(sd + n); // RN(1 / L(k,k).hi), or 0 where the quotient takes the plain form
+    __shared__ double2 slot[2];
+    const int j = blockIdx.x, tid = threadIdx.x;
+    L += blockIdx.y * sL;
+    X += blockIdx.y * sX;
+    for (int i = j + tid; i < n; i += T) {
+        const dd_t d = ld_dd(L + i + lda * (long)i);
+        dg[i] = make_double2(d.hi, d.lo);
+        rc[i] = mid_range(d.hi) && !all_ones(d.hi) ? __ddiv_rn(1.0, d.hi) : 0.0;
+        if (i + 1 < n) sd[i] = *reinterpret_cast<const double2 *>(L + i + 1 + lda * (long)i);
+    }
+    auto load = [&](int k, dd_t *f) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = j + tid + T * r;
+            f[r] = i > k && i < n ? ld_dd(L + i + lda * (long)k) : dd_zero(); // (i < n: k < n)
+        }
+    };
+    dd_t v[R], fa[R], fb[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = dd_from(tid + T * r == 0 ? 1.0 : 0.0);
+    load(j, fa);
+    load(j + 1, fb);
+    __syncthreads();
+    // entry k, and entry k+1 without step k's term, in every thread
+    dd_t cur = dd_from(1.0), nxt = dd_zero();
+    for (int k = j; k < n; ++k) {
+        const dd_t l = dd_make(dg[k].x, dg[k].y), s = k + 1 < n ? dd_make(sd[k].x, sd[k].y) : dd_zero();
+        const double y = rc[k];
+        const bool zero = dd_is_zero(cur);
+        dd_t x = dd_div_rest(cur, l, div_corrected(cur.hi, l.hi, y), y);
+        if (y == 0.0 || !mid_range(cur.hi)) x = zero ? cur : dd_div(cur, l);
+        const dd_t c = dd_sub(nxt, dd_mul(x, s));
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (j + T * r + T - 1 < k) continue; // rows above k
+            const int i = j + tid + T * r;
+            if (i == k) v[r] = x;
+            if (i > k && !zero) v[r] = dd_sub(v[r], dd_mul(x, fa[r]));
+            if (i == k + 2) slot[k & 1] = make_double2(v[r].hi, v[r].lo);
+            fa[r] = fb[r];
+        }
+        load(k + 2, fb);
+        __syncthreads();
+        cur = zero ? nxt : c;
+        nxt = dd_make(slot[k & 1].x, slot[k & 1].y); // (unused beyond the last row)
+    }
+    for (int i = tid; i < j; i += T) st_dd(X + i + ldx * (long)j, dd_zero());
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (j + tid + T * r < n) st_dd(X + j + tid + T * r + ldx * (long)j, v[r]);
+}
+template <int NW, int R> static void inv_rows_launch(cudaStream_t st, const dd_t *L, long lda, int n, dd_t *X, long ldx, int batch, long sL, long sX) {
+    const size_t smem = (2 * sizeof(double2) + sizeof(double)) * n;
+    inv_lower_rows_kernel<NW, R><<<dim3(n, batch), 32 * NW, smem, st>>>(L, lda, n, X, ldx, sL, sX);
+    CK_LAUNCH();
+}
+
 void inv_lower(cudaStream_t st, const dd_t *L, long lda, int n, dd_t *X, long ldx, int batch, long sL, long sX) {
     if (n <= 0 || batch <= 0) return;
     if (batch > MAX_GRID_YZ) {
@@ -1212,6 +1285,8 @@ void inv_lower(cudaStream_t st, const dd_t *L, long lda, int n, dd_t *X, long ld
         CK_LAUNCH();
         return;
     }
+    if (n <= 512) return inv_rows_launch<4, 4>(st, L, lda, n, X, ldx, batch, sL, sX);
+    if (n <= 1024) return inv_rows_launch<4, 8>(st, L, lda, n, X, ldx, batch, sL, sX);
     if (smem > 48 * 1024) CK(cudaFuncSetAttribute(inv_lower_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     inv_lower_kernel<<<dim3(n, batch), 128, smem, st>>>(L, lda, n, X, ldx, sL, sX);
     CK_LAUNCH();
