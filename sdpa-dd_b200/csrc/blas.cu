@@ -334,7 +334,7 @@ void gemm(cudaStream_t st, char ta, char tb, int mode, int M, int N, int K, cons
 // Hand-overs are named barriers; every one is reached by all its warps, a bad
 // pivot included.  Every entry sees x(i,j) -= L(j,k) L(i,k) for k ascending,
 // then the sqrt or the scaling.
-// Measured for nb = 64: 48 us; with warps that took turns at the pivot, on
+// Measured for nb = 64: 46 us; with warps that took turns at the pivot, on
 // lane 0 and with the plain divisions, behind an mbarrier a column, 70 us.
 // The same behind mbarriers 57 us (a wake-up costs several hundred cycles),
 // behind polled flags 53 us (the polls take the issue slots of the warps at
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_kernel(dd_t *A, long 
     else potrf_diag_body<0>(A + blockIdx.x * sA, lda, nb, c0, info, rdiag);
 }
 // CTA b: the block at column c0 of matrix b of a list (a kernel of its own:
-// with the block's order and pointers in registers it takes 66 us, not 48).
+// with the block's order and pointers in registers it takes 66 us, not 46).
 __global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_list_kernel(const PotrfItem *list, int c0) {
     const PotrfItem &it = list[blockIdx.x];
     if (c0 < it.n) potrf_diag_body<0>(it.A, it.n, min(POTRF_NB, it.n - c0), c0, it.info, it.rdiag);
