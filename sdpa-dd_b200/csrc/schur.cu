@@ -249,14 +249,9 @@ __global__ void schur_scatter_pairs_kernel(BlockView bv, int nfg, const dd_t *pa
 }
 
 // ----------------------------------------------------------- F3 owners
-// calF3 (sdpa_newton.cpp:937-977), one thread per pair.
-__global__ void schur_f3_kernel(BlockView bv, const int *ownF3, int nf3, const dd_t *X, const dd_t *invZ, dd_t *B, int m, dd_t *stage) {
-    const int r = blockIdx.y;
-    const int s_own = ownF3[r];
-    const int sp = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sp > s_own) return;
+// calF3 (sdpa_newton.cpp:937-977): the pair of sorted positions s_own, sp.
+__device__ __forceinline__ dd_t f3_pair(const BlockView &bv, int ti, int tj, const dd_t *X, const dd_t *invZ) {
     const int n = bv.n;
-    const int ti = bv.perm[s_own], tj = bv.perm[sp];
     const int oi = bv.coo_off[ti], ni = bv.nnz[ti], oj = bv.coo_off[tj], nj = bv.nnz[tj];
     const int *ri = bv.row + oi, *ci = bv.col + oi, *rj = bv.row + oj, *cj = bv.col + oj;
     const dd_t *vi = bv.val + oi, *vj = bv.val + oj;
@@ -282,7 +277,44 @@ __global__ void schur_f3_kernel(BlockView bv, const int *ownF3, int nf3, const d
         }
         ret = dd_acc(ret, dd_mul(v1, sum));
     }
-    pair_out(B, m, stage, bv.nc, s_own, sp, bv.con[ti], bv.con[tj], ret);
+    return ret;
+}
+// 32 owners x 32 partners a CTA, one thread for four pairs.  A pair is some 200
+// FP64 instructions and two entries of B, (i,j) and (j,i): the latter go out as
+// they are formed (neighbouring partners, neighbouring entries), the former
+// through shared memory with neighbouring owners side by side.  Staged pairs
+// (stage) lie partner by partner.
+// m = 9951 (one entry a constraint): 1.61 ms; a CTA of 128 partners an owner,
+// every (i,j) a line of its own, 2.57.
+constexpr int F3_T = 32;
+__global__ void __launch_bounds__(256) schur_f3_kernel(BlockView bv, const int *ownF3, int nf3, const dd_t *X, const dd_t *invZ, dd_t *B, int m, dd_t *stage) {
+    __shared__ double2 S[F3_T][F3_T + 1]; // owner, partner
+    const int tx = threadIdx.x % F3_T, ty = threadIdx.x / F3_T;
+    const int r0 = blockIdx.y * F3_T, sp0 = blockIdx.x * F3_T;
+    auto valid = [&](int r, int sp) { return r < nf3 && sp <= ownF3[r]; };
+    if (!__syncthreads_or(valid(r0 + tx, sp0))) return; // above every owner's last partner
+    for (int r = ty; r < F3_T; r += 256 / F3_T) {
+        if (!valid(r0 + r, sp0 + tx)) continue;
+        const int s_own = ownF3[r0 + r], sp = sp0 + tx, ti = bv.perm[s_own], tj = bv.perm[sp];
+        const dd_t v = f3_pair(bv, ti, tj, X, invZ);
+        if (stage) {
+            st_dd(stage + (long)s_own * bv.nc + sp, v);
+        } else {
+            S[r][tx] = make_double2(v.hi, v.lo);
+            dd_t *p = B + bv.con[tj] + (long)m * bv.con[ti];
+            st_dd(p, dd_acc(ld_dd(p), v));
+        }
+    }
+    if (stage) return;
+    __syncthreads();
+    for (int q = ty; q < F3_T; q += 256 / F3_T) {
+        if (!valid(r0 + tx, sp0 + q)) continue;
+        const int i = bv.con[bv.perm[ownF3[r0 + tx]]], j = bv.con[bv.perm[sp0 + q]];
+        if (i == j) continue;
+        const double2 v = S[tx][q];
+        dd_t *p = B + i + (long)m * j;
+        st_dd(p, dd_acc(ld_dd(p), dd_make(v.x, v.y)));
+    }
 }
 
 // One block's pairs, all on stream st, with F and G scratch of its own and
@@ -359,8 +391,8 @@ static void schur_block(Context &c, int l, cudaStream_t st, dd_t *Fb, dd_t *Gb, 
     }
     const int nf3 = bd.nF3();
     if (nf3 > 0) {
-        dim3 grid(ceil_div(bd.nsparse, 128), nf3);
-        schur_f3_kernel<<<grid, 128, 0, st>>>(bv, bd.ownF3.p, nf3, X, Zi, c.B.p, m, stage);
+        dim3 grid(ceil_div(bd.nsparse, F3_T), ceil_div(nf3, F3_T));
+        schur_f3_kernel<<<grid, 256, 0, st>>>(bv, bd.ownF3.p, nf3, X, Zi, c.B.p, m, stage);
         CK_LAUNCH();
     }
 }
