@@ -331,9 +331,15 @@ void gemm(cudaStream_t st, char ta, char tb, int mode, int M, int N, int K, cons
 // other sub-partitions hold columns 2 .. nb-1 in registers, in pairs j + j' =
 // nb + 2 whose nb - 2 entries fill two slots a lane, subtract the published
 // columns' terms, and hand column j over once column j - 2's term is in.
-// Hand-overs are named barriers; every one is reached by all its warps, a bad
-// pivot included.  Every entry sees x(i,j) -= L(j,k) L(i,k) for k ascending,
-// then the sqrt or the scaling.
+// Hand-overs are named barriers, which have no time limit: a warp that waits at
+// one is freed only by the other warps' arrivals, so no warp may leave by
+// itself.  The whole CTA decides on one read of *info whether it runs (other
+// CTAs of a batch write that word at any time); on a bad pivot k warp 0 still
+// publishes column k, so the helpers, which wait for published columns only, see
+// the stop there and end too (the hand-over of column k + 1, which its helper may
+// have signalled, is then waited for by nobody; an arrival does not wait).
+// Every entry sees x(i,j) -= L(j,k) L(i,k) for k ascending, then the sqrt or the
+// scaling.
 // Measured for nb = 64: 46 us; with warps that took turns at the pivot, on
 // lane 0 and with the plain divisions, behind an mbarrier a column, 70 us.
 // The same behind mbarriers 57 us (a wake-up costs several hundred cycles),
@@ -362,10 +368,12 @@ __device__ __forceinline__ void potrf_diag_body(dd_t *A, long lda, int nb_, int 
     const int nb = NB > 0 ? NB : nb_;
     extern __shared__ double2 sm[];
     double2 *S = sm; // nb x nb, column-major: columns on their way, then final
-    __shared__ int stop; // k + 1: bad pivot k
-    if (*info != 0) return;
+    __shared__ int skip, stop; // skip: a block before failed; stop: k + 1 for a bad pivot k
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) stop = 0;
+    if (tid == 0) {
+        skip = *reinterpret_cast<volatile int *>(info);
+        stop = 0;
+    }
     for (int e = tid; e < nb * nb; e += DIAG_THREADS) {
         const int i = e % nb, j = e / nb;
         if (i >= j) {
@@ -374,6 +382,7 @@ __device__ __forceinline__ void potrf_diag_body(dd_t *A, long lda, int nb_, int 
         }
     }
     __syncthreads();
+    if (skip != 0) return; // (written once: the same in every thread)
     volatile int *vstop = &stop;
     auto at = [&](int i, int j) {
         const double2 v = S[i + nb * j];
@@ -743,7 +752,7 @@ void potrf(cudaStream_t st, dd_t *A, long lda, int n, int *info_dev, dd_t *rdiag
 }
 
 int potrf_info_check(int info) {
-    if (info < 0) throw Error(ERR_CUDA, "potrf: a diagonal block's wait for one of its columns ran out");
+    if (info < 0) throw Error(ERR_CUDA, "potrf: a wait for a diagonal block's columns in the panel or the lookahead update ran out");
     return info;
 }
 

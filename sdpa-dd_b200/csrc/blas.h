@@ -29,15 +29,17 @@ void gemm_stacked(cudaStream_t st, bool rows, int n, int count, const dd_t *A, c
 // 'T' A c += alpha (sum_l A(l,i) B(l,j)).  op: 'N' or 'T'.
 void gemm_ab(cudaStream_t st, char ta, char tb, int M, int N, int K, dd_t alpha, const dd_t *A, long lda, const dd_t *B, long ldb, dd_t beta, dd_t *C,
              long ldc);
-// *info_dev = -1: a diagonal block's wait for one of its columns ran out
-// (the block is left as it was); potrf_info_check turns that into an error.
+// *info_dev = -1: a wait for a diagonal block's columns (in the panel below it
+// or the lookahead update of the next block) ran out; potrf_info_check turns
+// that into an error.
 void potrf(cudaStream_t st, dd_t *A, long lda, int n, int *info_dev, dd_t *rdiag_dev, OzakiWork *tc = nullptr);
 // Throws ERR_CUDA for a negative info (a wait that ran out); returns info.
 int potrf_info_check(int info);
 void zero_upper(cudaStream_t st, dd_t *A, long lda, int n, int batch = 1, long sA = 0);
 // Rpotrf("Lower") of `batch` matrices of order n <= 64, matrix b at A + b sA,
 // one CTA each (the single diagonal block of potrf); any failure sets
-// *info_dev to a failing column.
+// *info_dev, which all CTAs share, to a failing column, and matrices that start
+// later may be left as they were.
 void potrf_batched(cudaStream_t st, dd_t *A, long lda, int n, long sA, int batch, int *info_dev);
 // Rpotrf("Lower") of `count` matrices of orders up to nmax (a list in device
 // memory; leading dimension n, rdiag room for 64 reciprocals, info zero).
