@@ -984,7 +984,11 @@ template <bool FWD> __global__ void __launch_bounds__(TRSV_THREADS) trsv_wave_ke
     extern __shared__ double2 trsv_sm[];
     double2 *xs = trsv_sm + 2 * TRSV_B * TRSV_LD, *vs = xs + TRSV_B;
     double *rd = reinterpret_cast<double *>(vs + TRSV_B);
-    __shared__ int fail, zeros[2]; // zeros: some entry of the block's half is zero (forward: its steps are skipped)
+    // zeros: the zero entries of the block's halves (forward: their steps are
+    // skipped); two sets, since warps 0 and 1 read one while they subtract, each
+    // at its own pace, and write the next block's before the next barrier
+    __shared__ unsigned zeros[2][2];
+    __shared__ int fail;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     dd_t *x = a.x + a.ldx * blockIdx.y;
     int *flags = a.flags + (long)a.nblk * blockIdx.y;
@@ -1013,8 +1017,8 @@ template <bool FWD> __global__ void __launch_bounds__(TRSV_THREADS) trsv_wave_ke
                 } else {
                     const dd_t xa = tid < ib ? ldcg_dd(x + p * TRSV_B + tid) : dd_from(1.0);
                     xs[tid] = make_double2(xa.hi, xa.lo);
-                    const bool z = __any_sync(0xffffffffu, FWD && dd_is_zero(xa));
-                    if (lane == 0) zeros[warp] = z;
+                    const unsigned z = __ballot_sync(0xffffffffu, FWD && dd_is_zero(xa));
+                    if (lane == 0) zeros[u & 1][warp] = z;
                 }
             }
             __syncthreads(); // the tile and block p are in
@@ -1032,7 +1036,8 @@ template <bool FWD> __global__ void __launch_bounds__(TRSV_THREADS) trsv_wave_ke
             } else {
                 const double2 *at = FWD ? T + tid : T + TRSV_LD * tid;
                 const int st = FWD ? TRSV_LD : 1;
-                if (ib == TRSV_B && !(FWD && (zeros[0] || zeros[1]))) {
+                const unsigned zlo = zeros[u & 1][0], zhi = zeros[u & 1][1];
+                if (ib == TRSV_B && (zlo | zhi) == 0u) {
                     double2 z[2][8]; // the next eight products come while these are subtracted
 #pragma unroll
                     for (int q = 0; q < 8; ++q) z[0][q] = at[st * (FWD ? q : 63 - q)];
@@ -1047,7 +1052,7 @@ template <bool FWD> __global__ void __launch_bounds__(TRSV_THREADS) trsv_wave_ke
                 } else {
                     for (int q = 0; q < ib; ++q) {
                         const int t = FWD ? q : ib - 1 - q;
-                        if (FWD && xs[t].x == 0.0 && xs[t].y == 0.0) continue;
+                        if ((t < 32 ? zlo : zhi) >> (t & 31) & 1u) continue;
                         v = dd_sub(v, dd_make(at[st * t].x, at[st * t].y));
                     }
                 }
