@@ -196,13 +196,15 @@ __global__ void __launch_bounds__(T16_THREADS, T16_CTAS)
 // the work spreads over more SMs, and where the larger tiles would be mostly
 // padding (16 x 16 tiles run at about 0.7 of the FP64 rate, 64 x 64 at 0.9;
 // 200 products of order 20: 33 us in 64 x 64 tiles,
-// 9 in 16 x 16).  Each entry's k-order is the same either way.
+// 9 in 16 x 16).  A launch has at most MAX_GRID_YZ tiles down, 1,048,560 rows of
+// 16 x 16 tiles; taller products keep the 64 x 64 ones.  Each entry's k-order is
+// the same either way.
 constexpr long GEMM_SMALL_TILES = 74;
 template <bool TA, bool TB, int MODE>
 static void gemm_launch(cudaStream_t st, int M, int N, int K, const dd_t *A, long lda, long sA, const dd_t *B, long ldb, long sB, dd_t *C, long ldc,
                         long sC, int batch, bool lower, dd_t alpha = dd_t{1.0, 0.0}, dd_t beta = dd_t{1.0, 0.0}) {
     const long m16 = ceil_div(M, T16), n16 = ceil_div(N, T16), m64 = ceil_div(M, 64), n64 = ceil_div(N, 64);
-    if (m64 * n64 * batch < GEMM_SMALL_TILES || 13 * m16 * n16 < 10 * 16 * m64 * n64) {
+    if (m16 <= MAX_GRID_YZ && (m64 * n64 * batch < GEMM_SMALL_TILES || 13 * m16 * n16 < 10 * 16 * m64 * n64)) {
         dim3 grid((unsigned)n16, (unsigned)m16, batch);
         if (m16 * n16 * batch <= T16_PIPE_TILES)
             gemm16_kernel<TA, TB, MODE, true><<<grid, T16_THREADS, 0, st>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, lower ? 1 : 0, alpha, beta);
