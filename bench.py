@@ -589,7 +589,7 @@ def run_ours(args, world, rank, local):
         peaks = json.loads(pfile.read_text())
     if args.tc:
         t_ms, t_n = kern["potrf_trailing_update_tc"]
-        digits = (7 * args.tc + 7) // 8  # base-256 digits that carry the 7-bit slices
+        digits = (7 * args.tc + 1 + 7) // 8  # base-256 digits that carry the 7-bit slices
         pairs = digits * (digits + 1) // 2
         int8_ops = tr_fl * pairs  # entries x 64 (= tr_fl / 2) x pairs x 2 ops
         achieved = (int8_ops * args.steps) / (t_ms * 1e-3) / 1e12 if t_ms > 0 else None

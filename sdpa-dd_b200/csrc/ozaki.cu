@@ -4,15 +4,20 @@
 // e_r chosen so that every |P(r,k)| 2^-e_r <= 0.498, and written as a fixed
 // point number in B signed base-256 digits D_1 .. D_B in [-128, 127]:
 //   P(r,k) = 2^e_r sum_s D_s(r,k) 2^-8s  (+ remainder <= 2^-(8B+1) 2^e_r).
-// A caller's S 7-bit slices are carried by B = ceil(7S/8) digits (16 slices:
-// 14 digits, 112 bits and the rounding of the last one, as 16 7-bit digits
-// hold), so 105 digit products replace 136 and the diagonals are 14, not 16.
-// 0.498 < 127/255, the largest value that digits up to 127 reach.
+// 0.498 < 127/255, the largest value that digits up to 127 reach, so a row whose
+// largest entry lies in the top 0.4 % below a power of two takes a scale one bit
+// larger than 7-bit digits (in [-64, 64]) need.  A caller's S 7-bit slices are
+// therefore carried by B = ceil((7S + 1)/8) digits, so that every row keeps the
+// 7S bits below its largest entry (16 slices: 15 digits, truncated at 2^-120;
+// 120 digit products replace 136).  With 14 digits the error of such rows'
+// products was 3.6 times that of 16 7-bit digits (rms, small entries beside the
+// largest one: 2^-107.0 of the power of two against 2^-108.8); with 15 it is
+// 2^-113.9, at 5 % of the update's time.
 //
 // Products (ozaki_syrk_kernel).  C(i,j) -= 2^(e_i+e_j) sum_d 2^-8d A_d(i,j),
 // A_d = sum_{s+t=d} D_s(i,:) . D_t(j,:), for d = 2..B+1 (the B(B+1)/2 digit
 // pairs that reach 8(B+1) bits).  Every A_d is an exact int32 (|A_d| <=
-// (d-1) * 64 * 128 * 128 < 2^24), accumulated by tcgen05.mma kind::i8 in
+// (d-1) * 64 * 128 * 128 < 2^24, d <= 16), accumulated by tcgen05.mma kind::i8 in
 // tensor memory.
 //
 // One tcgen05.mma costs about the same time for any N up to 128 (on B200 a
@@ -22,18 +27,18 @@
 // stacked (row 16 (t-1) + j is digit t of column j), and its accumulators
 // are laid out by diagonal (diagonal d in columns 16 (d-2) .. 16 (d-2) + 15).
 // The MMA of A digit s against stacked B digits 1 .. B+1-s (N = 16 (B+1-s))
-// then writes diagonals s+1 .. B+1 in one instruction: B x 2 K steps = 28
-// MMAs per tile for 14 digits.
+// then writes diagonals s+1 .. B+1 in one instruction: B x 2 K steps = 30
+// MMAs per tile for 15 digits.
 //
-// Epilogue: an entry's diagonals combine exactly to one 128-bit integer; its
-// three 42-bit pieces become doubles scaled by 2^(e_i+e_j) and are summed with
+// Epilogue: an entry's diagonals combine exactly to four 64-bit integers
+// (oz_groups), which become doubles scaled by 2^(e_i+e_j) and are summed with
 // C's two halves (oz_sub).
 //
 // Kernel layout: one persistent CTA per SM over the tiles of the lower
 // triangle (row-block major, so a CTA keeps its 128-row A digits in shared
-// memory while it walks the columns).  Warp 17 stages everything with bulk
-// copies (cp.async.bulk, no multicast): B three tiles deep and C's tiles two
-// deep, a copy per column (clipped to the lower triangle).  Warp 0 lane 0
+// memory while it walks the columns).  Bulk copies (cp.async.bulk, no multicast)
+// stage everything: warp 17 the digits, B two tiles deep, and warp 18 C's tiles,
+// two deep, a copy per column (clipped to the lower triangle).  Warp 0 lane 0
 // issues the MMAs; warps 1-16 drain tensor memory, which holds two
 // accumulator buffers, so one tile multiplies while the last drains.
 // Operand layout in global memory: 16-row blocks, in a block digit by digit,
@@ -49,12 +54,12 @@
 // frees its tensor memory.
 //
 // What bounds it: C is read and written once per panel (32 bytes an entry of
-// the lower triangle, 0.24 ms at n = 9920) and a tile's 28 MMAs take about as
+// the lower triangle, 0.24 ms at n = 9920) and a tile's 30 MMAs take about as
 // long, but FP64 and tensor instructions wait for one another (see the
 // epilogue), so a tile takes the sum of the two.  Measured, one update: n =
-// 9920 448 us, n = 5000 133; with 16 7-bit digits assembled in FP64, C loaded
-// by the epilogue's threads and the copies issued by the MMA's thread 538 and
-// 157.
+// 9920 476 us, n = 5000 141, n = 2000 35; with 14 digits 454, 134 and 33.5; with
+// 16 7-bit digits assembled in FP64, C loaded by the epilogue's threads and the
+// copies issued by the MMA's thread 529, 154 and 33.
 #include "ozaki.h"
 
 #include <algorithm>
@@ -76,7 +81,7 @@ constexpr int OZ_MAX_REGS = 96;
 constexpr int OZ_A_BYTES = OZ_ROWS_A * OZ_K; // one digit of a 128-row block
 constexpr int OZ_B_BYTES = OZ_COLS_B * OZ_K; // one digit of a 16-row block
 constexpr int OZ_TILE_B = OZ_MAX_DIGITS * OZ_B_BYTES; // the stacked B digits of a tile
-constexpr int OZ_STAGES = 3;                 // B tiles in shared memory
+constexpr int OZ_STAGES = 2;                 // B tiles in shared memory
 constexpr int OZ_C_STAGES = 2;               // C tiles in shared memory
 constexpr int OZ_C_BYTES = OZ_ROWS_A * OZ_COLS_B * 16; // one C tile
 constexpr int OZ_ACC_COLS = 256; // tensor-memory columns of one accumulator buffer
@@ -341,15 +346,15 @@ __device__ __forceinline__ void tc_ld2(uint32_t taddr, int32_t *r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr));
 }
 
-// The diagonals of one entry, v[0..13] (diagonal d at v[d-2]; those beyond
+// The diagonals of one entry, v[0..14] (diagonal d at v[d-2]; those beyond
 // B+1 are zero), as four exact integers in units of 2^-40, 2^-72, 2^-104 and
-// 2^-136: A_2..A_5, A_6..A_9, A_10..A_13, A_14 and A_15.  |A_d| <= (d-1) 2^20,
-// so each is below 2^49.
+// 2^-136: A_2..A_5, A_6..A_9, A_10..A_13, A_14..A_16.  |A_d| <= (d-1) 2^20, so
+// each is below 2^49.
 __device__ __forceinline__ void oz_groups(const int32_t (*v)[2], int c, long long *w) {
 #pragma unroll
     for (int j = 0; j < 3; ++j)
         w[j] = (((long long)v[4 * j][c] * 16777216 + (long long)v[4 * j + 1][c] * 65536) + (long long)v[4 * j + 2][c] * 256) + v[4 * j + 3][c];
-    w[3] = (long long)v[12][c] * 16777216 + (long long)v[13][c] * 65536;
+    w[3] = ((long long)v[12][c] * 16777216 + (long long)v[13][c] * 65536) + (long long)v[14][c] * 256;
 }
 
 // The group w 2^e as a double: the bits of (2^52 + 2^51 + w) 2^e, then one
@@ -418,7 +423,7 @@ __device__ __noinline__ void oz_tile_far(uint32_t taddr, int nd, const double2 *
 // in the integer units (35 FP64 instructions an entry remain of 53), and an
 // accumulator buffer goes back only after the tile's FP64 part, not when it
 // is drained: the MMAs of the tile after next then run while the warps wait,
-// drain and join the next tile (n = 9920: 451 us against 494).
+// drain and join the next tile (n = 9920, 14 digits: 451 us against 494).
 // NDC: the digit count when known at compile time, else 0.
 template <int NDC>
 __device__ void oz_epilogue(const OzArgs &a, OzShared &S, const uint8_t *smC, int I, int J, int ntile) {
@@ -586,8 +591,8 @@ __device__ __forceinline__ void oz_transpose4(uint32_t a, uint32_t b, uint32_t c
 
 // Digits of 32 rows per CTA; warp c takes K bytes 16c..16c+15.  An entry is
 // a 120-bit fixed-point integer U = P(r,k) 2^(120-e); with 128 added to the
-// bytes of digits 1 .. nd and to the next lower one (the rounding of the last
-// digit), the bytes are the digits plus 128.
+// bytes of digits 1 .. nd and to the next lower one, if there is one (the rounding
+// of the last digit), the bytes are the digits plus 128.
 // A digit after the other peeled in dd arithmetic (10 FP64 operations each)
 // and written in two layouts took 14.6 us at n = 5003; this takes 6.8.
 __global__ void __launch_bounds__(128) ozaki_split_kernel(const dd_t *P, long ldp, int n, int k, int nd, int8_t *digits, int *exps) {

@@ -8,8 +8,10 @@
 namespace sddd {
 
 constexpr int OZ_MAX_SLICES = 16; // 7-bit slices a caller may ask for
-// base-256 digits that carry `slices` 7-bit slices in the trailing update
-constexpr int ozaki_digits(int slices) { return (7 * slices + 7) / 8; }
+// Base-256 digits that carry `slices` 7-bit slices in the trailing update: one
+// bit more than the slices have, since rows whose largest entry lies just below a
+// power of two take a scale one bit larger than 7-bit digits need (ozaki.cu).
+constexpr int ozaki_digits(int slices) { return (7 * slices + 1 + 7) / 8; }
 constexpr int OZ_MAX_DIGITS = ozaki_digits(OZ_MAX_SLICES);
 constexpr int OZ_K = 64;        // panel width the split handles (K of the update)
 constexpr int OZ_ROWS_A = 128;  // output tile rows (MMA M)
