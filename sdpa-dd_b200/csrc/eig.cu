@@ -355,7 +355,10 @@ void launch_lanczos(cudaStream_t st, const int *ids, int nb, int nsp, long maxn,
         if (!ok) cudaGetLastError();
         most[dev & 63] = ok ? LZ_CLUSTER : 8;
     }
-    const int R = lanczos_cluster(maxn, nb * nsp, most[dev & 63]);
+    // The split of the sums, and so a value's last bits, follow the cluster's
+    // size; sized for two spaces in either case, so that an eigenvalue asked for
+    // alone is the one that the solver's launch over both spaces gives.
+    const int R = lanczos_cluster(maxn, 2 * nb, most[dev & 63]);
     const bool smem = lanczos_smem(maxn, R, true) <= SMEM_MAX;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(nb * nsp * R));
