@@ -358,7 +358,11 @@ void launch_lanczos(cudaStream_t st, const int *ids, int nb, int nsp, long maxn,
     // The split of the sums, and so a value's last bits, follow the cluster's
     // size; sized for two spaces in either case, so that an eigenvalue asked for
     // alone is the one that the solver's launch over both spaces gives.
-    const int R = lanczos_cluster(maxn, 2 * nb, most[dev & 63]);
+    // A CTA's own rows of two vectors are in shared memory in either form, so a
+    // large block among many small ones needs a larger cluster than their number
+    // asks for (one CTA holds 6200 rows).
+    int R = lanczos_cluster(maxn, 2 * nb, most[dev & 63]);
+    while (R < most[dev & 63] && lanczos_smem(maxn, R, false) > SMEM_MAX) R *= 2;
     const bool smem = lanczos_smem(maxn, R, true) <= SMEM_MAX;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(nb * nsp * R));
