@@ -149,8 +149,9 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
         }
 }
 
-// The same in 16 x 16 tiles (tile16.cuh).  Order 500: 183 us, the FP64 work
-// alone 134; one entry a thread, 256 threads, took 204.
+// The same in 16 x 16 tiles (tile16.cuh).  Order 500: 183 us in isolation, the
+// FP64 work alone 134; one entry a thread, 256 threads, took 204 (a call of that
+// order, with its launch and wait, 224 and 228).
 template <bool TA, bool TB, int MODE, bool PIPE>
 __global__ void __launch_bounds__(T16_THREADS, T16_CTAS)
     gemm16_kernel(int M, int N, int K, const dd_t *__restrict__ A, long lda, long sA, const dd_t *__restrict__ B, long ldb, long sB, dd_t *C, long ldc,
@@ -239,9 +240,10 @@ template <int TS> static void stacked_launch(cudaStream_t st, bool rows, int n, 
 }
 void gemm_stacked(cudaStream_t st, bool rows, int n, int count, const dd_t *A, const dd_t *B, dd_t *C) {
     if (n <= 0 || count <= 0) return;
-    // the fewest warps over the short dimension, then the fewest tiles
+    // the fewest warps over the short dimension, then the fewest tiles (an odd
+    // width has as many warps as the next even one)
     int ts = 8, best = 1 << 30;
-    for (int t = 16; t >= 8; --t) {
+    for (int t = 16; t >= 8; t -= 2) {
         const int tiles = (int)ceil_div(n, 4 * t), cost = tiles * (int)ceil_div(16 * t, 32);
         if (cost < best) best = cost, ts = t;
     }
@@ -252,13 +254,9 @@ void gemm_stacked(cudaStream_t st, bool rows, int n, int count, const dd_t *A, c
     }
     switch (ts) {
     case 8: stacked_launch<8>(st, rows, n, count, A, B, C); break;
-    case 9: stacked_launch<9>(st, rows, n, count, A, B, C); break;
     case 10: stacked_launch<10>(st, rows, n, count, A, B, C); break;
-    case 11: stacked_launch<11>(st, rows, n, count, A, B, C); break;
     case 12: stacked_launch<12>(st, rows, n, count, A, B, C); break;
-    case 13: stacked_launch<13>(st, rows, n, count, A, B, C); break;
     case 14: stacked_launch<14>(st, rows, n, count, A, B, C); break;
-    case 15: stacked_launch<15>(st, rows, n, count, A, B, C); break;
     default: stacked_launch<16>(st, rows, n, count, A, B, C);
     }
 }
