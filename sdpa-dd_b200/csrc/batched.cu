@@ -279,7 +279,7 @@ CoreEngine::CoreEngine(int device) : p(new Impl) {
     // shape between event-record nodes (recorded as external events, so
     // that every launch of the graph records them and the autotuner can
     // time the shapes; a plain record inside a capture only orders the
-    // graph), the factorisations
+    // graph); the factorisations follow it (potrf_list)
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
     core_zero_kernel<<<dim3(8, CORE_CAP), 256, 0, p->stream>>>(p->db);
